@@ -1055,12 +1055,17 @@ static tfv_config single_step_config(const tfv_config* cfg) {
 
 int tfv_step_workspace_size(const tfv_config* cfg, int32_t precision, size_t* bytes) {
   if (!cfg || !bytes) return fail(TFV_EINVAL, "invalid arguments");
+  // with and without a per-cell gamma: the tail split of the tiles follows the
+  // resident CTAs of the kernel, which differ between the two
   tfv_config c = single_step_config(cfg);
-  tfv_batch* b = nullptr;
-  const int r = create_internal(cfg->dim, precision, 1, &c, nullptr, true, &b);
-  if (r) return r;
-  *bytes = b->total;
-  tfv_batch_destroy(b);
+  *bytes = 0;
+  for (const bool varg : {false, true}) {
+    tfv_batch* b = nullptr;
+    const int r = create_internal(cfg->dim, precision, 1, &c, nullptr, varg, &b);
+    if (r) return r;
+    *bytes = std::max(*bytes, b->total);
+    tfv_batch_destroy(b);
+  }
   return TFV_OK;
 }
 

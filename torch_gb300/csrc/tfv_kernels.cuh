@@ -317,6 +317,7 @@ struct HydroSmem {
   static constexpr int kXo = 16 / (int)sizeof(R);
   int tx, ty, pw, ph, bw, bh, xo, nthreads;
   size_t slot_elems;  // elements per ring slot (128-byte multiple)
+  int goff;           // element of a slot where its gamma plane starts
   size_t ring_off, bar_off, box_off, fa_off, fb_off, bs_off, red_off, items_off, bytes;
   __host__ __device__ void init(int tx_, int ty_) {
     tx = tx_;
@@ -327,7 +328,10 @@ struct HydroSmem {
     ph = DIM == 3 ? ty + 4 : 1;
     bw = tx + 2;
     bh = DIM == 3 ? ty + 2 : 1;
-    slot_elems = ((size_t)NL * ph * pw * sizeof(R) + 127) / 128 * 128 / sizeof(R);
+    // each tensor copy lands on a 128-byte boundary: the state at the slot's
+    // start, gamma (VARG) at the next boundary after the NV state planes
+    goff = (int)(((size_t)NV * ph * pw * sizeof(R) + 127) / 128 * 128 / sizeof(R));
+    slot_elems = (((size_t)goff + (size_t)(NL - NV) * ph * pw) * sizeof(R) + 127) / 128 * 128 / sizeof(R);
     size_t o = 0;
     ring_off = o;  // dynamic shared memory starts 128-byte aligned
     o += sizeof(R) * 3 * slot_elems;
@@ -381,10 +385,11 @@ struct HydroTile {
         const int lb = row - c * h;
         const R* srow = (VARG && c == NV) ? gam + base + (int64_t)lb * g.na
                                           : U + c * g.cs + base + (int64_t)lb * g.na;
-        R* drow = dst + c * plane + lb * S.pw + (S.xo - 2);
+        const int at = (VARG && c == NV ? S.goff : c * plane) + lb * S.pw + (S.xo - 2);
+        R* drow = dst + at;
         for (int la = lane; la < w; la += 32) {
           if (!TFV_IN(3, base + (int64_t)lb * g.na + la, g.cs) ||
-              !TFV_IN(4, c * plane + lb * S.pw + (S.xo - 2) + la, (int64_t)S.slot_elems))
+              !TFV_IN(4, at + la, (int64_t)S.slot_elems))
             continue;
           drow[la] = srow[la];
         }
@@ -393,9 +398,10 @@ struct HydroTile {
       for (int row = threadIdx.x >> 5; row < nrows; row += nwarps) {
         const int c = row / h;
         const int lb = row - c * h;
-        R* drow = dst + c * plane + lb * S.pw + (S.xo - 2);
+        const int at = (VARG && c == NV ? S.goff : c * plane) + lb * S.pw + (S.xo - 2);
+        R* drow = dst + at;
         for (int la = lane; la < w; la += 32) {
-          if (!TFV_IN(5, c * plane + lb * S.pw + (S.xo - 2) + la, (int64_t)S.slot_elems)) continue;
+          if (!TFV_IN(5, at + la, (int64_t)S.slot_elems)) continue;
           drow[la] = fetch_padded<R, DIM>(d, g, U, VARG ? gam : (const R*)nullptr, c, x0 - 2 + la,
                                           DIM == 3 ? y0 - 2 + lb : 0, p);
         }
@@ -435,8 +441,9 @@ struct HydroTile {
         la = aL + (q - row * wm);
         lb = row < bL ? row : (by + 4 - bR) + (row - bL);
       }
-      if (!TFV_IN(6, c * cplane + lb * S.pw + la + (S.xo - 2), (int64_t)S.slot_elems)) continue;
-      dst[c * cplane + lb * S.pw + la + (S.xo - 2)] = fetch_padded<R, DIM>(
+      const int at = (VARG && c == NV ? S.goff : c * cplane) + lb * S.pw + la + (S.xo - 2);
+      if (!TFV_IN(6, at, (int64_t)S.slot_elems)) continue;
+      dst[at] = fetch_padded<R, DIM>(
           d, g, U, VARG ? gam : (const R*)nullptr, c, x0 - 2 + la, DIM == 3 ? y0 - 2 + lb : 0, p);
     }
   }
@@ -471,7 +478,7 @@ __device__ __forceinline__ void cell_stage(const R* ringm, const R* ringc, const
     return;
   }
 #endif
-  const R g = VARG ? ringc[NV * plane + li] : gconst;
+  const R g = VARG ? ringc[S.goff + li] : gconst;
 
   R u[NV];
 #pragma unroll
@@ -708,10 +715,10 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
         mbar_expect_tx(bar, box_bytes + gbox_bytes);
         if (DIM == 3) {
           tma_load_4d(dst, map_u, x0 - S.xo, y0 - 2, p, 0, bar);
-          if (VARG) tma_load_3d(dst + NV * cplane, map_g, x0 - S.xo, y0 - 2, p, bar);
+          if (VARG) tma_load_3d(dst + S.goff, map_g, x0 - S.xo, y0 - 2, p, bar);
         } else {
           tma_load_3d(dst, map_u, x0 - S.xo, p, 0, bar);
-          if (VARG) tma_load_2d(dst + NV * cplane, map_g, x0 - S.xo, p, bar);
+          if (VARG) tma_load_2d(dst + S.goff, map_g, x0 - S.xo, p, bar);
         }
       }
     } else {
@@ -878,8 +885,8 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
         if (VARG) {
           const int li = kind == 0 ? (DIM == 3 ? (j + 2) * S.pw : 0) + i - 1 + S.xo
                                    : (j + 1) * S.pw + i + S.xo;
-          gl = rc[NV * cplane + li];
-          gr = rc[NV * cplane + li + (kind == 0 ? 1 : S.pw)];
+          gl = rc[S.goff + li];
+          gr = rc[S.goff + li + (kind == 0 ? 1 : S.pw)];
         }
         if constexpr (Exact<R>::value || DIM != 3)
           hllc<R, NV - 3>(ul, ur, gl, gr, f);
@@ -941,7 +948,7 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
     for (int c = 0; c < NV; ++c) Fm[c] = R(0);
     if (owner) {
       const int li = (DIM == 3 ? (ob + 2) * S.pw : 0) + oa + S.xo;
-      const R gcur = VARG ? rc[NV * cplane + li] : gconst;
+      const R gcur = VARG ? rc[S.goff + li] : gconst;
       if (it >= p0) {
         if constexpr (Exact<R>::value || DIM != 3)
           hllc_cartesian<R, NV>(Tprev, Bn, gprev, gcur, MD, Fm);
