@@ -1,5 +1,7 @@
-"""Per-cell gamma staged by tensor copies."""
-
+"""Default tilings against explicit ones, and per-cell gamma staged by tensor
+copies.  Per-cell arithmetic does not depend on the tile shape, so states of
+the default tiling (double precision: chosen by a cost model; 1D: 122 cells in
+128 threads) equal those of another tiling bit for bit."""
 
 import numpy as np
 import pytest
@@ -38,3 +40,38 @@ def test_2d_fp32_step_with_gamma_per_cell():
     got = stepfn.muscl_hancock_step_2d(u, *args, precision="fp32")
     for c in range(4):
         assert np.abs(got[c] - want[c]).mean() <= 1e-5 * np.abs(want[c]).mean()
+
+
+@pytest.mark.parametrize("counts,tile", [
+    ((31, 7), (128, 1, 32)), ((62, 5), (32, 1, 4)), ((126, 33), (128, 1, 32)),
+    ((250, 18), (64, 1, 16)), ((2, 2), (128, 1, 32)),
+    ((15, 9, 5), (32, 4, 32)), ((28, 16, 33), (16, 8, 16)), ((14, 14, 2), (32, 4, 32)),
+    ((29, 43, 17), (32, 4, 32)),
+])
+@pytest.mark.parametrize("boundary", ["Open", "Reflective", "Periodic"])
+def test_fp64_default_tiling_equals_explicit_tiles(counts, tile, boundary):
+    dim = len(counts)
+    states = []
+    for t in (None, tile):
+        sim = torch_gb300.Simulation(rough(counts), [1.0] * dim, t_end=1.0, limiter="Superbee",
+                                     boundaries=[boundary] * dim, tile=t)
+        for _ in range(3):
+            sim.step()
+        states.append((sim.state, sim.time))
+    np.testing.assert_array_equal(states[0][0], states[1][0])
+    assert states[0][1] == states[1][1]
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("n", [5, 121, 122, 123, 245, 1000])
+def test_1d_default_tiling_equals_whole_warp_tiles(n, precision):
+    for boundary in ("Open", "Reflective", "Periodic"):
+        states = []
+        for t in (None, (256, 1, 1)):
+            sim = torch_gb300.Simulation(rough((n,)), [1.0], t_end=1.0, limiter="VanLeer",
+                                         boundaries=[boundary], precision=precision, tile=t)
+            for _ in range(5):
+                sim.step()
+            states.append((sim.state, sim.time))
+        np.testing.assert_array_equal(states[0][0], states[1][0])
+        assert states[0][1] == states[1][1]

@@ -30,6 +30,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I" + str(IN
 F32 = ["-fmad=true", "-ftz=true", "-prec-div=false", "-prec-sqrt=false"]
 UNITS = {
     "tfv_f64.cu": ["-fmad=false"],
+    "tfv_f64_3d.cu": ["-fmad=false"],
     "tfv_f32_3d.cu": F32,
     "tfv_f32_2d.cu": F32,
     "tfv_host.cu": [],

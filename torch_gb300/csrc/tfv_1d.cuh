@@ -64,15 +64,15 @@ __device__ __forceinline__ R gamma1(const InstDesc& d, const R* gam, int k) {
 // uconsv_to_uprim (torchSolver.py:117-127)
 template <typename R>
 __device__ __forceinline__ void prim1(const R* u, R g, R& rho, R& v, R& p) {
-  rho = np_max(u[0], R(kFloor));
-  v = u[1] / rho;
-  p = np_max((u[2] - (R(0.5) * rho) * (v * v)) * (g - R(1)), R(kFloor));
+  rho = floored(u[0]);
+  v = qd(u[1], rho);
+  p = floored((u[2] - hf(rho) * (v * v)) * (g - R(1)));
 }
 
 // sound_speed_calc (torchSolver.py:81-87)
 template <typename R>
 __device__ __forceinline__ R sound1(R rho, R p, R g) {
-  return sqrt((g * np_max(p, R(0))) / np_max(rho, R(kFloor)));
+  return rt(qd(g * np_max(p, R(0)), floored(rho)));
 }
 
 // u_to_fu_calc (torchSolver.py:145-156)
@@ -96,27 +96,29 @@ __device__ __forceinline__ void waves1(const InstDesc& d, const R* L, const R* R
   const R al = sound1(rl, pl, gl), ar = sound1(rr, pr, gr);
   R sl, sr;
   if (d.wavespeed == 0) {  // Pressure Based (PVRS)
-    const R rho_avg = R(0.5) * (rr + rl);
-    const R a_avg = R(0.5) * (al + ar);
-    const R ps = np_max(R(0), R(0.5) * (pl + pr) - ((R(0.5) * (ur - ul)) * rho_avg) * a_avg);
-    const R ql = ps > pl ? sqrt(R(1) + ((gl + R(1)) / (R(2) * gl)) * (ps / pl - R(1))) : R(1);
-    const R qr = ps > pr ? sqrt(R(1) + ((gr + R(1)) / (R(2) * gr)) * (ps / pr - R(1))) : R(1);
+    const R rho_avg = hf(rr + rl);
+    const R a_avg = hf(al + ar);
+    const R ps = np_max(R(0), hf(pl + pr) - (hf(ur - ul) * rho_avg) * a_avg);
+    const R ql = lt_(pl, ps)
+                     ? rt(R(1) + qd(gl + R(1), tw(gl)) * (qd(ps, pl) - R(1))) : R(1);
+    const R qr = lt_(pr, ps)
+                     ? rt(R(1) + qd(gr + R(1), tw(gr)) * (qd(ps, pr) - R(1))) : R(1);
     sl = ul - al * ql;
     sr = ur + ar * qr;
   } else {  // Enthalpy Based (Roe-Einfeldt)
-    const R el = rl * (R(0.5) * (ul * ul) + pl / ((gl - R(1)) * rl));
-    const R er = rr * (R(0.5) * (ur * ur) + pr / ((gr - R(1)) * rr));
-    const R sql = sqrt(rl), sqr = sqrt(rr);
-    const R den = np_max(sql + sqr, R(kFloor));
-    const R uavg = (sql * ul + sqr * ur) / den;
-    const R havg = (sql * ((el + pl) / rl) + sqr * ((er + pr) / rr)) / den;
-    const R gavg = R(0.5) * (gl + gr);
-    const R aavg = sqrt(np_max((gavg - R(1)) * (havg - R(0.5) * (uavg * uavg)), R(1e-10)));
+    const R el = rl * (hf(ul * ul) + qd(pl, (gl - R(1)) * rl));
+    const R er = rr * (hf(ur * ur) + qd(pr, (gr - R(1)) * rr));
+    const R sql = rt(rl), sqr = rt(rr);
+    const R den = floored(sql + sqr);
+    const R uavg = qd(sql * ul + sqr * ur, den);
+    const R havg = qd(sql * qd(el + pl, rl) + sqr * qd(er + pr, rr), den);
+    const R gavg = hf(gl + gr);
+    const R aavg = rt(max_pos((gavg - R(1)) * (havg - hf(uavg * uavg)), R(1e-10)));
     sl = np_min(ul - al, uavg - aavg);
     sr = np_max(ur + ar, uavg + aavg);
   }
   const R den = guarded(rl * (sl - ul) - rr * (sr - ur), R(kGuard));
-  R ss = (((pr - pl) + (rl * ul) * (sl - ul)) - (rr * ur) * (sr - ur)) / den;
+  R ss = qd(((pr - pl) + (rl * ul) * (sl - ul)) - (rr * ur) * (sr - ur), den);
   ss = np_min(np_max(ss, sl), sr);
   s[0] = sl;
   s[1] = ss;
@@ -125,39 +127,47 @@ __device__ __forceinline__ void waves1(const InstDesc& d, const R* L, const R* R
 
 // Sweby-bounded limited slope (python/cfdSolver/torchSolver.py:201-275).
 template <typename R>
-__device__ __forceinline__ R nan0(R x) { return isfinite(x) ? x : R(0); }
+__device__ __forceinline__ R nan0(R x) { return finite_(x) ? x : R(0); }
+// nan0(a / b): a zero divisor (quiescent gas) gives an infinity or NaN, so 0
+template <typename R>
+__device__ __forceinline__ R nan0_quotient(R a, R b) {
+  if constexpr (Exact<R>::value) {
+    if (((s64_hi(b) << 1) | s64_lo(b)) == 0u) return R(0);
+  }
+  return nan0(qd(a, b));
+}
 
 template <typename R>
 __device__ __forceinline__ R limit1(R delta, R uw, R dw, R w, int limiter) {
-  const R r = nan0(uw / dw);
+  const R r = nan0_quotient(uw, dw);
   const R denom = (R(1) - w) + (R(1) + w) * r;
-  const R eps_r = nan0(R(2) / (fabs(denom) < R(kFloor) ? R(kFloor) : denom));
+  const R eps_r = nan0(qd(R(2), guarded(denom, R(kFloor))));
   R eps = R(0);
   switch (limiter) {
     case 1:  // Albada
-      if (r > R(0)) eps = np_min(nan0((r * (R(1) + r)) / (R(1) + r * r)), eps_r);
+      if (gt0(r)) eps = np_min(nan0(qd(r * (R(1) + r), R(1) + r * r)), eps_r);
       break;
     case 2:  // MINBEE
-      if (r > R(0) && r < R(1)) eps = r;
-      if (r >= R(1)) eps = np_min(R(1), eps_r);
+      if (gt0(r) && lt_(r, R(1))) eps = r;
+      if (le_(R(1), r)) eps = np_min(R(1), eps_r);
       break;
     case 3:  // Superbee
-      if (r > R(0))
-        eps = np_min(nan0(np_max(R(0), np_max(np_min(R(2) * r, R(1)), np_min(r, R(2))))), eps_r);
+      if (gt0(r))
+        eps = np_min(nan0(np_max(R(0), np_max(np_min(tw(r), R(1)), np_min(r, R(2))))), eps_r);
       break;
     case 4:  // Unos
-      eps = np_min(np_max(R(0), np_min(np_min(R(2), R(2) * r), (R(2) + r) / R(3))), eps_r);
+      eps = np_min(np_max(R(0), np_min(np_min(R(2), tw(r)), qd(R(2) + r, R(3)))), eps_r);
       break;
     default:  // VanLeer
-      if (r > R(0)) eps = np_min(nan0((R(2) * r) / (R(1) + r)), eps_r);
+      if (gt0(r)) eps = np_min(nan0(qd(tw(r), R(1) + r)), eps_r);
       break;
   }
   eps = np_max(R(0), nan0(eps));
   const R slope = eps * delta;
-  const R bound = R(2) * np_min(fabs(uw), fabs(dw));
-  if (!(uw * dw > R(0))) return R(0);
+  const R bound = tw(np_min(fabs(uw), fabs(dw)));
+  if (!gt0(uw * dw)) return R(0);
   const R mag = np_min(fabs(slope), bound);
-  return dw > R(0) ? mag : -mag;
+  return gt0(dw) ? mag : -mag;
 }
 
 // HLLC with precomputed S_L, S_R (python/cfdSolver/torchSolver.py:534-676).
@@ -167,25 +177,25 @@ __device__ __forceinline__ void hllc1(const InstDesc& d, const R* UL, const R* U
   R rl, vl, pl, rr, vr, pr;
   prim1(UL, gl, rl, vl, pl);
   prim1(UR, gr, rr, vr, pr);
-  const R el = rl * (R(0.5) * (vl * vl) + pl / ((gl - R(1)) * rl));
-  const R er = rr * (R(0.5) * (vr * vr) + pr / ((gr - R(1)) * rr));
+  const R el = rl * (hf(vl * vl) + qd(pl, (gl - R(1)) * rl));
+  const R er = rr * (hf(vr * vr) + qd(pr, (gr - R(1)) * rr));
   R fl[3], fr[3];
   flux1(UL, gl, fl);
   flux1(UR, gr, fr);
   const R den = guarded(rl * (sl - vl) - rr * (sr - vr), R(kGuard));
-  R ss = (((pr - pl) + (rl * vl) * (sl - vl)) - (rr * vr) * (sr - vr)) / den;
+  R ss = qd(((pr - pl) + (rl * vl) * (sl - vl)) - (rr * vr) * (sr - vr), den);
   ss = np_min(np_max(ss, sl), sr);
   const R eps = R(kFloor);
   R fls[3], frs[3];
   if (d.variant == 0) {  // Variante 1 - Original
-    const bool okl = fabs(sl - ss) > eps, okr = fabs(sr - ss) > eps;
+    const bool okl = gt_pos(fabs(sl - ss), eps), okr = gt_pos(fabs(sr - ss), eps);
     const R dl = okl ? sl - ss : -eps;
     const R dr = okr ? sr - ss : eps;
-    const R dul = fabs(sl - vl) < eps ? -eps : sl - vl;
-    const R dur = fabs(sr - vr) < eps ? eps : sr - vr;
-    const R tl = el / rl + (ss - vl) * (ss + pl / (rl * dul));
-    const R tr = er / rr + (ss - vr) * (ss + pr / (rr * dur));
-    const R kl = rl * ((sl - vl) / dl), kr = rr * ((sr - vr) / dr);
+    const R dul = abs_lt(sl - vl, eps) ? -eps : sl - vl;
+    const R dur = abs_lt(sr - vr, eps) ? eps : sr - vr;
+    const R tl = qd(el, rl) + (ss - vl) * (ss + qd(pl, rl * dul));
+    const R tr = qd(er, rr) + (ss - vr) * (ss + qd(pr, rr * dur));
+    const R kl = rl * qd(sl - vl, dl), kr = rr * qd(sr - vr, dr);
     const R stl[3] = {kl * R(1), kl * ss, kl * tl};
     const R str[3] = {kr * R(1), kr * ss, kr * tr};
 #pragma unroll
@@ -195,25 +205,27 @@ __device__ __forceinline__ void hllc1(const InstDesc& d, const R* UL, const R* U
     }
   } else {  // Variante_2
     const R ds[3] = {R(0), R(1), ss};
-    const R sgl = (sl - ss + R(1e-30)) > R(0) ? R(1) : ((sl - ss + R(1e-30)) < R(0) ? R(-1) : R(0));
-    const R sgr = (sr - ss + R(1e-30)) > R(0) ? R(1) : ((sr - ss + R(1e-30)) < R(0) ? R(-1) : R(0));
-    const R dl = fabs(sl - ss) < eps ? sgl * eps : sl - ss;
-    const R dr = fabs(sr - ss) < eps ? sgr * eps : sr - ss;
+    const R gl_ = sl - ss + R(1e-30), gr_ = sr - ss + R(1e-30);
+    const R sgl = gt0(gl_) ? R(1) : (lt0(gl_) ? R(-1) : R(0));
+    const R sgr = gt0(gr_) ? R(1) : (lt0(gr_) ? R(-1) : R(0));
+    const R dl = abs_lt(sl - ss, eps) ? sgl * eps : sl - ss;
+    const R dr = abs_lt(sr - ss, eps) ? sgr * eps : sr - ss;
     const R ml = sl * (pl + (rl * (sl - vl)) * (ss - vl));
     const R mr = sr * (pr + (rr * (sr - vr)) * (ss - vr));
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      fls[c] = (ss * (sl * UL[c] - fl[c]) + ml * ds[c]) / dl;
-      frs[c] = (ss * (sr * UR[c] - fr[c]) + mr * ds[c]) / dr;
+      fls[c] = qd(ss * (sl * UL[c] - fl[c]) + ml * ds[c], dl);
+      frs[c] = qd(ss * (sr * UR[c] - fr[c]) + mr * ds[c], dr);
     }
   }
+  const bool m0 = gt0(sl), m1 = le0(sl) && gt0(ss), m2 = le0(ss) && ge0(sr), m3 = lt0(sr);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     R v = R(0);
-    if (sl > R(0)) v = fl[c];
-    if (sl <= R(0) && ss > R(0)) v = fls[c];
-    if (ss <= R(0) && sr >= R(0)) v = frs[c];
-    if (sr < R(0)) v = fr[c];
+    if (m0) v = fl[c];
+    if (m1) v = fls[c];
+    if (m2) v = frs[c];
+    if (m3) v = fr[c];
     out[c] = v;
   }
 }
@@ -282,7 +294,7 @@ __global__ void __launch_bounds__(256) waves1d_kernel(StepArgs A, int in_step) {
           if (!TFV_IN(41, f, n + 1)) continue;
           if (!TFV_INSIDE(62, S.waves + k * (n + 1) + f, d.scratch, S.flux + 3 * (n + 1))) continue;
           S.waves[k * (n + 1) + f] = s[k];
-          ws = fmax(ws, fabs(s[k]));
+          ws = run_max(ws, fabs(s[k]));
         }
       }
       R u[3];
@@ -320,7 +332,7 @@ __global__ void __launch_bounds__(256) waves1d_kernel(StepArgs A, int in_step) {
 // between neighbours cm and cp (python/cfdSolver/torchSolver.py:412-491).
 template <typename R>
 __device__ __forceinline__ R recon1_coef(const InstDesc& d, const InstState& st) {
-  return -R(st.dt / (2.0 * d.h[0]));  // -(dt / (2 dx)) of the Hancock half step
+  return -R(soft_div(st.dt, soft_twice(d.h[0])));  // -(dt / (2 dx)) of the Hancock half step
 }
 
 // kcoef = recon1_coef(d, st), formed once per tile by the caller
@@ -332,16 +344,17 @@ __device__ __forceinline__ void recon1_cells(const InstDesc& d, const R* c0, con
     R rho, v, p;
     prim1(c0, g, rho, v, p);
     const R a = sound1(rho, p, g);
-    const R mach = nan0(fabs(v) / np_max(a, R(kFloor)));
-    w = np_min(np_max((R(1) - mach) / (R(1) + mach), R(-1)), R(1));
+    const R mach = nan0(qd(fabs(v), floored(a)));
+    w = np_min(np_max(qd(R(1) - mach, R(1) + mach), R(-1)), R(1));
   }
   R ul[3], ur[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const R delta = R(0.5) * (cp[c] - cm[c]);
+    const R delta = hf(cp[c] - cm[c]);
     const R lim = limit1(delta, c0[c] - cm[c], cp[c] - c0[c], w, d.limiter);
-    ul[c] = c0[c] - R(0.5) * lim;
-    ur[c] = c0[c] + R(0.5) * lim;
+    const R half = hf(lim);
+    ul[c] = c0[c] - half;
+    ur[c] = c0[c] + half;
   }
   R fl[3], fr[3];
   flux1(ul, g, fl);
@@ -355,9 +368,11 @@ __device__ __forceinline__ void recon1_cells(const InstDesc& d, const R* c0, con
   R* outs[2] = {ol, orr};
   for (int sidx = 0; sidx < 2; ++sidx) {
     R* s = outs[sidx];
-    const R p = (g - R(1)) * (s[2] - (R(0.5) * (s[1] * s[1])) / np_max(s[0], R(kFloor)));
-    const bool badc = s[0] <= R(kFloor) || p <= R(kFloor) || !isfinite(s[0]) ||
-                      !isfinite(s[1]) || !isfinite(s[2]);
+    const R p = (g - R(1)) * (s[2] - qd(hf(s[1] * s[1]), floored(s[0])));
+    // not above the floor (a NaN pressure alone keeps the state, as the
+    // reference's comparison does)
+    const bool badc = le_(s[0], R(kFloor)) || le_(p, R(kFloor)) || !finite_(s[0]) ||
+                      !finite_(s[1]) || !finite_(s[2]);
     if (badc)
       for (int c = 0; c < 3; ++c) s[c] = c0[c];
   }
@@ -435,7 +450,7 @@ __device__ __forceinline__ void face_flux1(const InstDesc& d, const R* U, const 
   flux1(L, gl, pfl);
   flux1(Rr, gr, pfr);
 #pragma unroll
-  for (int c = 0; c < 3; ++c) F[c] = R(0.5) * ((pfl[c] + pfr[c]) - alpha * (Rr[c] - L[c]));
+  for (int c = 0; c < 3; ++c) F[c] = hf((pfl[c] + pfr[c]) - alpha * (Rr[c] - L[c]));
 }
 
 template <typename R, bool VARG>
@@ -705,13 +720,13 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
       if (fl_r) Rr[1] = -Rr[1];
       waves1(d, L, Rr, gamma1(d, gam, f - 1), gamma1(d, gam, f), w3);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) ws = fmax(ws, fabs(w3[k]));
+      for (int k = 0; k < 3; ++k) ws = run_max(ws, fabs(w3[k]));
       if (s < ax) {
         R rho, v, p;
         const R g = gamma1(d, gam, f);
         R uc[3] = {un_s[0 * TS + s + 1], un_s[1 * TS + s + 1], un_s[2 * TS + s + 1]};
         prim1(uc, g, rho, v, p);
-        wh = fmax(wh, fabs(v) + sound1(rho, p, g));
+        wh = run_max(wh, fabs(v) + sound1(rho, p, g));
       }
     }
     const int fl = block_or(bad ? kFlagNonphysical : 0, reinterpret_cast<int*>(red));

@@ -158,10 +158,11 @@ int resident_slots(const tfv_batch* b) {
   const bool f64 = b->precision == TFV_FP64;
   int per_sm = 0;
   if (b->dim == 3)
-    per_sm = f64 ? occupancy3_f64(b->varg, b->tile.tx, b->tile.ty)
-                 : occupancy3_f32(b->varg, b->tile.tx, b->tile.ty);
+    per_sm = f64 ? occupancy3_f64(b->varg, b->tile.tx, b->tile.ty, b->block)
+                 : occupancy3_f32(b->varg, b->tile.tx, b->tile.ty, b->block);
   else
-    per_sm = f64 ? occupancy2_f64(b->varg, b->tile.tx) : occupancy2_f32(b->varg, b->tile.tx);
+    per_sm = f64 ? occupancy2_f64(b->varg, b->tile.tx, b->block)
+                 : occupancy2_f32(b->varg, b->tile.tx, b->block);
   cudaGetLastError();
   return per_sm > 0 ? per_sm * sms : 0;
 }
@@ -459,8 +460,8 @@ cudaError_t checked_sync(const tfv_batch* b, int op, int lim, int t0, int t1, cu
                  op, lim, t0, t1, b->dim, b->precision, b->n, cudaGetErrorString(e));
     return e;
   }
-  cudaError_t (*readers[3])(unsigned long long*) = {check_read_f64, check_read_f32_3d,
-                                                    check_read_f32_2d};
+  cudaError_t (*readers[4])(unsigned long long*) = {check_read_f64, check_read_f64_3d,
+                                                    check_read_f32_3d, check_read_f32_2d};
   for (auto rd : readers) {
     unsigned long long rec[4] = {0, 0, 0, 0};
     e = rd(rec);
@@ -619,6 +620,111 @@ int tfv_batch_create(int32_t dim, int32_t precision, int32_t n, const tfv_config
   return create_internal(dim, precision, n, cfgs, tile, false, out);
 }
 
+// SMs of the current device; the target chip's count where there is no device
+// (a plan made on a host without one is only sized, never launched).
+static int device_sms() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    cudaGetLastError();
+    sms = 152;
+  }
+  return sms;
+}
+
+// Tile of a double-precision 2D / 3D batch: the shape and chunk of the list
+// with the smallest modelled time.  Shapes leave lanes for the ring cells
+// (30 + 2, 62 + 2, 126 + 2 in 2D; 10 x 8 + 40 of 128 and 14 x 14 + 60 of 256
+// threads in 3D), so no warp does a second cell stage per plane; their widths
+// are even, as the 16-byte tensor-copy boundary asks.  A warp's plane costs
+// one cell stage, its share of the in-plane faces and one marching face
+// (cell stage / face: 1 in 2D, 2.7 in 3D); a chunk of c planes takes c + 2
+// stages, c in-plane rounds and c + 1 marching faces.  A unit of that work
+// takes alpha per wave of 16 resident warps (latency of the integer
+// sequences) plus beta per resident warp of the SM (FP64 pipe), in
+// microseconds measured on the GB300: alpha 6.6, beta 0.95 in 2D; 1.2 and
+// 1.18 in 3D (cell stage and three faces overlap there).  Few-row chunks win
+// on small grids (256^2: 136 us per step with 30 x 2 against 761 with 128 x 32
+// whose 16 tiles leave most SMs idle), long ones on large grids (1024^2: 1.05
+// ms with 126 x 16, 1.26 with 30 x 4).
+static void fp64_tile(tfv_batch* b, const tfv_config* cfgs) {
+  struct Shape {
+    int tx, ty, threads;
+  };
+  static const Shape k2d[] = {{30, 1, 32}, {62, 1, 64}, {126, 1, 128}};
+  static const Shape k3d[] = {{10, 8, 128}, {14, 14, 256}};
+  static const int kChunks[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
+  const bool d3 = b->dim == 3;
+  const Shape* shapes = d3 ? k3d : k2d;
+  const int nshapes = d3 ? 2 : 3;
+  const double sms = device_sms();
+  const double stage = d3 ? 2.7 : 1.0, alpha = d3 ? 1.2 : 6.6, beta = d3 ? 1.18 : 0.95;
+  double best = 0.0;
+  for (int k = 0; k < nshapes; ++k) {
+    const Shape& S = shapes[k];
+    const double faces = double((S.tx + 1) * S.ty + (d3 ? S.tx * (S.ty + 1) : 0)) / S.threads;
+    for (int c : kChunks) {
+      double tiles = 0.0;
+      for (int i = 0; i < b->n; ++i) {
+        const int32_t* n = cfgs[i].counts;
+        tiles += std::ceil(double(n[0]) / S.tx) * (d3 ? std::ceil(double(n[1]) / S.ty) : 1.0) *
+                 std::ceil(double(n[d3 ? 2 : 1]) / c);
+      }
+      const double warps = std::ceil(tiles / sms) * (S.threads / 32);
+      const double units = (c + 2) * stage + c * faces + (c + 1);
+      const double t = units * (alpha * std::ceil(warps / 16.0) + beta * warps);
+      if (best == 0.0 || t < best) {
+        best = t;
+        b->tile.tx = S.tx;
+        b->tile.ty = S.ty;
+        b->tile.chunk = c;
+        b->block = S.threads;
+      }
+    }
+  }
+}
+
+static void default_tile(tfv_batch* b, const tfv_config* cfgs) {
+  // FP32 3D: 16 x 16 (three CTAs per SM; the fastest measured shape at 256^3),
+  // 40-plane chunks (256^3: 1.065 ms per step kernel against 1.105 with 32 and
+  // 1.085 with 48, measured).
+  // FP32 2D: rows of 124 cells in 128 threads (the two ring cells on the
+  // spare lanes: no warp does a second cell stage or face per row), 32-row
+  // chunks (4096^2: 31.9 G cell-updates/s against 29.8 for 128 x 32; 64-row
+  // chunks reach 32.5 there but leave small grids too few tiles: the
+  // autotuner tries them per batch).
+  b->tile.persistent_ctas = 0;
+  b->tile.tma = 1;
+  b->tile.ty = 1;
+  b->tile.chunk = 32;
+  if (b->dim == 1) {
+    // 122 cells in 128 threads: the tile and its 3-cell halo are one item per
+    // thread in every phase of the step (256 cells in 256 threads took two
+    // rounds: 16 tubes of 194k cells, FP32 40.1 -> 34.4 us per step, FP64 204 ->
+    // 156; one 1000-cell tube, FP64 59.6 -> 38.6)
+    b->tile.tx = 122;
+    b->block = 128;
+  } else if (b->precision == TFV_FP64) {
+    fp64_tile(b, cfgs);
+  } else if (b->dim == 3) {
+    b->tile.tx = b->tile.ty = 16;
+    b->tile.chunk = 40;
+  } else {
+    b->tile.tx = 124;
+  }
+}
+
+// The largest tiles: the smallest workspace (tfv_hydro_step_static).
+static tfv_tile compact_tile(int32_t dim, int32_t precision) {
+  const bool f32 = precision == TFV_FP32;
+  tfv_tile t{};
+  t.tx = dim == 3 ? (f32 ? 16 : 32) : (dim == 2 ? (f32 ? 124 : 128) : 256);
+  t.ty = dim == 3 ? (f32 ? 16 : 4) : 1;
+  t.chunk = dim == 3 && f32 ? 40 : 32;
+  t.tma = 1;
+  return t;
+}
+
 static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_config* cfgs,
                            const tfv_tile* tile, bool varg, tfv_batch** out) {
   if (!out || !cfgs || n < 1) return fail(TFV_EINVAL, "invalid arguments");
@@ -649,21 +755,7 @@ static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_
   if (tile) {
     b->tile = *tile;
   } else {
-    // 3D: 32 x 4 (FP64, one CTA per SM) or 16 x 16 (FP32, three CTAs per SM;
-    // the fastest measured shape at 256^3)
-    // 2D FP32: rows of 124 cells in 128 threads (the two ring cells on the
-    // spare lanes: no warp does a second cell stage or face per row), 32-row
-    // chunks (4096^2: 31.9 G cell-updates/s against 29.8 for 128 x 32; 64-row
-    // chunks reach 32.5 there but leave small grids too few tiles: the
-    // autotuner tries them per batch)
-    const bool f32 = precision == TFV_FP32;
-    b->tile.tx = dim == 3 ? (f32 ? 16 : 32) : (dim == 2 ? (f32 ? 124 : 128) : 256);
-    b->tile.ty = dim == 3 ? (f32 ? 16 : 4) : 1;
-    // 3D FP32: 40-plane chunks (256^3: 1.065 ms per step kernel against 1.105
-    // with 32 and 1.085 with 48, measured)
-    b->tile.chunk = dim == 3 && f32 ? 40 : 32;
-    b->tile.persistent_ctas = 0;
-    b->tile.tma = 1;
+    default_tile(b, cfgs);
   }
   if (dim != 3) b->tile.ty = 1;
   {
@@ -677,13 +769,16 @@ static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_
     }
   }
   if (b->tile.tx < 4 || b->tile.ty < 1 || b->tile.chunk < 1 || b->tile.tx * b->tile.ty > 256 ||
-      step_threads(dim, precision == TFV_FP64, b->tile.tx, b->tile.ty) % 32 != 0) {
+      (tile && step_threads(dim, precision == TFV_FP64, b->tile.tx, b->tile.ty) % 32 != 0)) {
     delete b;
     return fail(TFV_EINVAL,
                 "tile shape must have tx >= 4, ty >= 1, chunk >= 1, at most 256 cells, and "
                 "tx*ty a multiple of 32 (single precision: tx*ty plus its ring cells within "
                 "whole warps of at most 256 threads)");
   }
+  // every kernel of the batch runs whole warps (the block reductions shuffle
+  // over full warps); lanes past a tile's cells own nothing
+  if (b->block == 0) b->block = step_threads(dim, precision == TFV_FP64, b->tile.tx, b->tile.ty);
   b->reactive = cfgs[0].reactive != 0;
   // reactive SI closure: gamma(lambda) per cell, computed into the workspace
   b->own_gamma = b->reactive && cfgs[0].closure == TFV_CLOSURE_SI;
@@ -823,9 +918,6 @@ int tfv_batch_bind(tfv_batch* b, void* workspace, void* const* states, void* con
   A.fin_slices = b->fin_slices;
   A.ws_lo = b->ws;
   A.ws_hi = b->ws + b->total;
-  // every kernel of the batch runs whole warps (the block reductions shuffle
-  // over full warps); lanes past a tile's cells own nothing
-  b->block = step_threads(b->dim, b->precision == TFV_FP64, b->tile.tx, b->tile.ty);
   b->grid = grid_for(b, A.ntiles);
   TFV_CUDA(cudaMemcpyAsync(b->ws + b->off_desc, b->desc.data(), sizeof(InstDesc) * b->n,
                            cudaMemcpyHostToDevice, b->stream));
@@ -1053,15 +1145,15 @@ static tfv_config single_step_config(const tfv_config* cfg) {
   return c;
 }
 
-int tfv_step_workspace_size(const tfv_config* cfg, int32_t precision, size_t* bytes) {
-  if (!cfg || !bytes) return fail(TFV_EINVAL, "invalid arguments");
+static int step_workspace(const tfv_config* cfg, int32_t precision, const tfv_tile* tile,
+                          size_t* bytes) {
   // with and without a per-cell gamma: the tail split of the tiles follows the
   // resident CTAs of the kernel, which differ between the two
   tfv_config c = single_step_config(cfg);
   *bytes = 0;
   for (const bool varg : {false, true}) {
     tfv_batch* b = nullptr;
-    const int r = create_internal(cfg->dim, precision, 1, &c, nullptr, varg, &b);
+    const int r = create_internal(cfg->dim, precision, 1, &c, tile, varg, &b);
     if (r) return r;
     *bytes = std::max(*bytes, b->total);
     tfv_batch_destroy(b);
@@ -1069,14 +1161,20 @@ int tfv_step_workspace_size(const tfv_config* cfg, int32_t precision, size_t* by
   return TFV_OK;
 }
 
-int tfv_hydro_step(const tfv_config* cfg, int32_t precision, const void* state_in,
-                   void* state_out, const void* gamma_cells, double dt, void* fx, void* fy,
-                   void* fz, void* workspace, int32_t* used_fallback, void* stream) {
+int tfv_step_workspace_size(const tfv_config* cfg, int32_t precision, size_t* bytes) {
+  if (!cfg || !bytes) return fail(TFV_EINVAL, "invalid arguments");
+  return step_workspace(cfg, precision, nullptr, bytes);
+}
+
+static int hydro_step(const tfv_config* cfg, int32_t precision, const tfv_tile* tile,
+                      const void* state_in, void* state_out, const void* gamma_cells, double dt,
+                      void* fx, void* fy, void* fz, void* workspace, int32_t* used_fallback,
+                      void* stream) {
   if (!cfg || !state_in || !state_out || !workspace) return fail(TFV_EINVAL, "invalid arguments");
   if (!(std::isfinite(dt) && dt >= 0)) return fail(TFV_EINVAL, "dt must be finite and >= 0");
   tfv_config c = single_step_config(cfg);
   tfv_batch* b = nullptr;
-  int r = create_internal(cfg->dim, precision, 1, &c, nullptr, gamma_cells != nullptr, &b);
+  int r = create_internal(cfg->dim, precision, 1, &c, tile, gamma_cells != nullptr, &b);
   if (r) return r;
   b->desc[0].gam = const_cast<void*>(gamma_cells);
   void* ring[2] = {const_cast<void*>(state_in), state_out};
@@ -1107,6 +1205,13 @@ int tfv_hydro_step(const tfv_config* cfg, int32_t precision, const void* state_i
   }
   tfv_batch_destroy(b);
   return r;
+}
+
+int tfv_hydro_step(const tfv_config* cfg, int32_t precision, const void* state_in,
+                   void* state_out, const void* gamma_cells, double dt, void* fx, void* fy,
+                   void* fz, void* workspace, int32_t* used_fallback, void* stream) {
+  return hydro_step(cfg, precision, nullptr, state_in, state_out, gamma_cells, dt, fx, fy, fz,
+                    workspace, used_fallback, stream);
 }
 
 }  // extern "C"
@@ -1141,8 +1246,17 @@ extern "C" int tfv_hydro_step_static(const tfv_config* cfg, int32_t precision,
                                      void* fz, int32_t* used_fallback, void* stream) {
   if (!cfg) return fail(TFV_EINVAL, "invalid arguments");
   size_t need = 0;
-  int r = tfv_step_workspace_size(cfg, precision, &need);
+  int r = step_workspace(cfg, precision, nullptr, &need);
   if (r) return r;
+  // a grid whose default tiling asks for more scratch takes the largest tiles
+  // (fewer of them; values do not depend on the tile shape)
+  tfv_tile compact;
+  const tfv_tile* tile = nullptr;
+  if (need > kStaticScratchBytes) {
+    compact = compact_tile(cfg->dim, precision);
+    tile = &compact;
+    if ((r = step_workspace(cfg, precision, tile, &need))) return r;
+  }
   if (need > kStaticScratchBytes)
     return fail(TFV_EINVAL, "this grid needs " + std::to_string(need) +
                                 " bytes of step scratch but tfv_hydro_step_static holds " +
@@ -1151,6 +1265,6 @@ extern "C" int tfv_hydro_step_static(const tfv_config* cfg, int32_t precision,
   void* ws = nullptr;
   r = static_scratch(&ws);
   if (r) return r;
-  return tfv_hydro_step(cfg, precision, state_in, state_out, gamma_cells, dt, fx, fy, fz, ws,
-                        used_fallback, stream);
+  return hydro_step(cfg, precision, tile, state_in, state_out, gamma_cells, dt, fx, fy, fz, ws,
+                    used_fallback, stream);
 }

@@ -113,7 +113,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
+  for (int o = 16; o > 0; o >>= 1) v = soft_fmax_run(v, __shfl_down_sync(0xffffffffu, v, o));
   return v;
 }
 __device__ __forceinline__ float warp_max(float v) {
@@ -150,7 +150,7 @@ __device__ __forceinline__ double block_max(double v, double* scratch) {
   __syncthreads();
   double t = 0.0;
   if (threadIdx.x == 0) {
-    for (int w = 0; w < nw; ++w) t = fmax(t, scratch[w]);
+    for (int w = 0; w < nw; ++w) t = soft_fmax_run(t, scratch[w]);
   }
   return t;
 }
@@ -319,10 +319,10 @@ struct HydroSmem {
   size_t slot_elems;  // elements per ring slot (128-byte multiple)
   int goff;           // element of a slot where its gamma plane starts
   size_t ring_off, bar_off, box_off, fa_off, fb_off, bs_off, red_off, items_off, bytes;
-  __host__ __device__ void init(int tx_, int ty_) {
+  __host__ __device__ void init(int tx_, int ty_, int threads) {
     tx = tx_;
     ty = DIM == 3 ? ty_ : 1;
-    nthreads = step_threads(DIM, Exact<R>::value, tx, ty);
+    nthreads = threads;
     xo = kXo;
     pw = tx + 2 * kXo;
     ph = DIM == 3 ? ty + 4 : 1;
@@ -449,6 +449,10 @@ struct HydroTile {
   }
 };
 
+// Half of a stored slope: the double-precision cell stage stores halves.
+__device__ __forceinline__ double half_slope(double s) { return s; }
+__device__ __forceinline__ float half_slope(float s) { return 0.5f * s; }
+
 // Cell stage at local position (a, b) of the current plane: limited slopes in
 // every direction and the Hancock predictor (python/cfdSolver/torchSolver3D.py:
 // 135-151, python/cfdSolver/torchSolver2D.py:305-377).  Writes predictor and
@@ -503,12 +507,14 @@ __device__ __forceinline__ void cell_stage(const R* ringm, const R* ringc, const
         up = ringc[c * plane + li + S.pw];
       }
       s[c] = limited_slope<R, DIM, LIM>(um, u[c], up);
+      // double precision keeps the half slope (exact): every use is a half
+      if constexpr (Exact<R>::value) s[c] = hf(s[c]);
     }
     R vp[NV], vm[NV], fp[NV], fm[NV];
 #pragma unroll
     for (int c = 0; c < NV; ++c) {
-      vp[c] = u[c] + R(0.5) * s[c];
-      vm[c] = u[c] - R(0.5) * s[c];
+      vp[c] = u[c] + half_slope(s[c]);
+      vm[c] = u[c] - half_slope(s[c]);
     }
     if (DIM == 3) {
       flux3<R>(vp, g, dd + 1, fp);
@@ -540,10 +546,10 @@ __device__ __forceinline__ void cell_stage(const R* ringm, const R* ringc, const
   }
   if (DIM == 2) {
     // predictor floors (python/cfdSolver/torchSolver2D.py:367-377)
-    ubar[0] = np_max(ubar[0], R(kFloor));
-    const R ke = (R(0.5) * (ubar[1] * ubar[1] + ubar[2] * ubar[2])) / ubar[0];
+    ubar[0] = floored(ubar[0]);
+    const R ke = qd(hf(ubar[1] * ubar[1] + ubar[2] * ubar[2]), ubar[0]);
     const R pb = (g - R(1)) * (ubar[3] - ke);
-    if (pb < R(kFloor)) ubar[3] = R(kFloor) / (g - R(1)) + ke;
+    if (lt_(pb, R(kFloor))) ubar[3] = qd(R(kFloor), g - R(1)) + ke;
   }
 #pragma unroll
   for (int c = 0; c < NV; ++c) bub[c * bplane + bi] = ubar[c];
@@ -557,10 +563,10 @@ __device__ __forceinline__ void cell_stage(const R* ringm, const R* ringc, const
       for (int c = 0; c < NV; ++c) {
         const R s = dd == 0 ? bsa[c * bplane + bi]
                             : (dd == 1 ? bsb[c * bplane + bi] : smarch[c]);
-        lo[c] = ubar[c] + R(-0.5) * s;
-        hi[c] = ubar[c] + R(0.5) * s;
+        lo[c] = ubar[c] - half_slope(s);
+        hi[c] = ubar[c] + half_slope(s);
       }
-      ok = ok && physical_cell<R, NV>(lo) && physical_cell<R, NV>(hi);
+      ok = ok & physical_cell<R, NV>(lo) & physical_cell<R, NV>(hi);
     }
     if (!ok) gate = true;
   }
@@ -575,10 +581,11 @@ __device__ __forceinline__ void wave_speeds(const R* u, R g, R* w) {
     const R rho = u[0];
     const R s = (u[1] * u[1] + u[2] * u[2]) + u[3] * u[3];
     if constexpr (Exact<R>::value) {
-      const R p = (g - R(1)) * (u[4] - (R(0.5) * s) / rho);
-      const R a = sqrt((g * p) / rho);
+      const Divisor<R> dr(rho);
+      const R p = (g - R(1)) * (u[4] - qd(hf(s), dr));
+      const R a = rt(qd(g * p, dr));
 #pragma unroll
-      for (int k = 0; k < 3; ++k) w[k] = fabs(u[k + 1] / rho) + a;
+      for (int k = 0; k < 3; ++k) w[k] = fabs(qd(u[k + 1], dr)) + a;
     } else {
       const R irho = rcp(rho);
       const R p = (g - R(1)) * (u[4] - R(0.5) * s * irho);
@@ -588,16 +595,18 @@ __device__ __forceinline__ void wave_speeds(const R* u, R g, R* w) {
     }
   } else if (DIM == 1) {
     // hydro_dt_1d: uconsv_to_uprim + sound_speed_calc (pressure floored at 0)
-    const R rho = np_max(u[0], R(kFloor));
-    const R v = u[1] / rho;
-    const R p = np_max((u[2] - (R(0.5) * rho) * (v * v)) * (g - R(1)), R(kFloor));
-    w[0] = fabs(v) + sqrt((g * np_max(p, R(0))) / np_max(rho, R(kFloor)));
+    const R rho = floored(u[0]);
+    const Divisor<R> dr(rho);
+    const R v = qd(u[1], dr);
+    const R p = floored((u[2] - hf(rho) * (v * v)) * (g - R(1)));
+    w[0] = fabs(v) + rt(qd(g * p, dr));  // floored already (NaN propagates)
   } else {
-    const R rho = np_max(u[0], R(kFloor));
-    const R vx = u[1] / rho;
-    const R vy = u[2] / rho;
-    const R p = np_max((g - R(1)) * (u[3] - (R(0.5) * rho) * (vx * vx + vy * vy)), R(kFloor));
-    const R a = sqrt((g * np_max(p, R(kFloor))) / np_max(rho, R(kFloor)));
+    const R rho = floored(u[0]);
+    const Divisor<R> dr(rho);
+    const R vx = qd(u[1], dr);
+    const R vy = qd(u[2], dr);
+    const R p = floored((g - R(1)) * (u[3] - hf(rho) * (vx * vx + vy * vy)));
+    const R a = rt(qd(g * p, dr));
     w[0] = fabs(vx) + a;
     w[1] = fabs(vy) + a;
   }
@@ -853,8 +862,8 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
       if (k < 0) {
 #pragma unroll
         for (int c = 0; c < NV; ++c) {
-          Bn[c] = ub[c] - R(0.5) * sm[c];
-          Tn[c] = ub[c] + R(0.5) * sm[c];
+          Bn[c] = ub[c] - half_slope(sm[c]);
+          Tn[c] = ub[c] + half_slope(sm[c]);
         }
       }
     }
@@ -878,8 +887,8 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
 #pragma unroll
         for (int c = 0; c < NV; ++c) {
           const int cc = (kind == 1 && c == 1) ? 2 : ((kind == 1 && c == 2) ? 1 : c);
-          ul[c] = bub[cc * bplane + bl] + R(0.5) * bsl[cc * bplane + bl];
-          ur[c] = bub[cc * bplane + br] - R(0.5) * bsl[cc * bplane + br];
+          ul[c] = bub[cc * bplane + bl] + half_slope(bsl[cc * bplane + bl]);
+          ur[c] = bub[cc * bplane + br] - half_slope(bsl[cc * bplane + br]);
         }
         R gl = gconst, gr = gconst;
         if (VARG) {
@@ -972,7 +981,7 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
           R w[DIM];
           wave_speeds<R, DIM>(un, gprev, w);
 #pragma unroll
-          for (int k = 0; k < DIM; ++k) wmax[k] = fmax(wmax[k], w[k]);
+          for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
         }
 #pragma unroll
         for (int c = 0; c < NV; ++c) Fprev[c] = Fm[c];
@@ -1038,7 +1047,7 @@ __global__ void __launch_bounds__(256, TFV_HYDRO_MIN_BLOCKS) hydro_kernel(StepAr
   // would hide the address space and turn every shared access generic)
   unsigned char* smem = smem_raw + ((128u - (smem_u32(smem_raw) & 127u)) & 127u);
   HydroSmem<R, DIM, VARG> S;
-  S.init(TX > 0 ? TX : A.tx, TY > 0 ? TY : A.ty);
+  S.init(TX > 0 ? TX : A.tx, TY > 0 ? TY : A.ty, blockDim.x);
   if (threadIdx.x == 0) {
     uint64_t* bars = smem_at<uint64_t>(smem, S.bar_off);
     for (int k = 0; k < 3; ++k) mbar_init(bars + k, 1);
@@ -1211,7 +1220,7 @@ __global__ void __launch_bounds__(256) fallback_kernel(StepArgs A) {
         R w[DIM];
         wave_speeds<R, DIM>(un, gc, w);
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) wmax[k] = fmax(wmax[k], w[k]);
+        for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
       }
     }
     int fl = block_or(bad ? kFlagNonphysical : 0, reinterpret_cast<int*>(red));
@@ -1292,7 +1301,7 @@ __global__ void __launch_bounds__(256) waves_kernel(StepArgs A, int sums) {
           R w[DIM];
           wave_speeds<R, DIM>(u[q], gc[q], w);
 #pragma unroll
-          for (int k = 0; k < DIM; ++k) wmax[k] = fmax(wmax[k], w[k]);
+          for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
         }
       }
     }
@@ -1326,8 +1335,8 @@ __global__ void __launch_bounds__(256) waves_kernel(StepArgs A, int sums) {
 // hydro estimates (w[0] = max |S|, w[1] = max(|u| + a)).
 __device__ __forceinline__ double cfl_dt(const InstDesc& d, const double* w) {
   if (d.dim == 3) {
-    const double total = (w[0] / d.h[0] + w[1] / d.h[1]) + w[2] / d.h[2];
-    return d.cfl / total;
+    const double total = (soft_div(w[0], d.h[0]) + soft_div(w[1], d.h[1])) + soft_div(w[2], d.h[2]);
+    return soft_div(d.cfl, total);
   }
   if (d.dim == 2) {
     double w0 = w[0], w1 = w[1];
@@ -1339,12 +1348,13 @@ __device__ __forceinline__ double cfl_dt(const InstDesc& d, const double* w) {
       w0 = fmax(w0, fabs(ux) + a);
       w1 = fmax(w1, fabs(vy) + a);
     }
-    const double total = w0 / d.h[0] + w1 / d.h[1];
-    return total <= 1e-12 ? 1e-3 : d.cfl / total;
+    const double total = soft_div(w0, d.h[0]) + soft_div(w1, d.h[1]);
+    return soft_le(total, 1e-12) ? 1e-3 : soft_div(d.cfl, total);
   }
-  const double dw = w[0] > 0 ? (d.cfl * d.h[0]) / w[0] : 1e-6;
-  const double dh = d.cfl * d.h[0] / w[1];
-  return dh < dw ? dh : dw;
+  const double ch = d.cfl * d.h[0];
+  const double dw = soft_gt0(w[0]) ? soft_div(ch, w[0]) : 1e-6;
+  const double dh = soft_div(ch, w[1]);
+  return soft_lt(dh, dw) ? dh : dw;
 }
 
 __device__ __forceinline__ void set_dt(const InstDesc& d, InstState& st, double dt) {
@@ -1394,22 +1404,23 @@ __device__ __forceinline__ void plan_next_warp(const InstDesc& d, InstState& st,
   }
   double dt;
   if (d.dim == 3) {
-    const double q = lane < 3 ? w[lane] / d.h[lane] : 0.0;
+    const double q = lane < 3 ? soft_div(w[lane], d.h[lane]) : 0.0;
     const double q0 = __shfl_sync(0xffffffffu, q, 0);
     const double q1 = __shfl_sync(0xffffffffu, q, 1);
     const double q2 = __shfl_sync(0xffffffffu, q, 2);
     const double total = (q0 + q1) + q2;
-    dt = d.cfl / total;
+    dt = soft_div(d.cfl, total);
   } else {
     dt = cfl_dt(d, w);
   }
   if (fp32) dt = (double)(float)dt;
   const double rem = d.t_end - st.time;
   if (rem < dt) dt = rem;
-  if (lane < 3) {
-    st.coef_half[lane] = (0.5 * dt) / d.h[lane];
-  } else if (lane < 6) {
-    st.coef_full[lane - 3] = dt / d.h[lane - 3];
+  if (lane < 6) {  // one division per lane: dt / h_d and half of dt over h_d
+    const int k = lane < 3 ? lane : lane - 3;
+    const double c = soft_div(lane < 3 ? soft_half(dt) : dt, d.h[k]);
+    if (lane < 3) st.coef_half[k] = c;
+    else st.coef_full[k] = c;
   } else if (lane == 6) {
     st.dt = dt;
     st.status = (!isfinite(dt) || dt <= 0.0 || st.time + dt == st.time) ? kErrStall : kReady;
@@ -1429,7 +1440,7 @@ __device__ __forceinline__ float texp(float x) { return expf(x); }
 
 template <typename R>
 __device__ __forceinline__ R gamma_of_lambda(R lam) {
-  return (R(4.5) - lam) / (R(3.5) - lam);
+  return qd(R(4.5) - lam, R(3.5) - lam);
 }
 
 // Chemistry constants of an instance in the arithmetic type, converted once
@@ -1448,20 +1459,19 @@ __device__ __forceinline__ R reaction_rate(const Chem<R>& d, R lam, R s0, R s1, 
   const bool si = d.closure == 0;
   const R g = si ? gamma_of_lambda(lam) : d.gamma;
   // uconsv_to_uprim (torchSolver.py:117-127)
-  const R rho = np_max(s0, R(kFloor));
-  const R u = s1 / rho;
-  const R p = np_max((s2 - (R(0.5) * rho) * (u * u)) * (g - R(1)), R(kFloor));
+  const R rho = floored(s0);
+  const R u = qd(s1, rho);
+  const R p = floored((s2 - hf(rho) * (u * u)) * (g - R(1)));
   R t;
   if (si) {
-    // temp_calc (torchSolver.py:90-114)
-    const R rho2 = np_max(rho, R(kFloor));
+    // temp_calc (torchSolver.py:90-114); rho is floored already
     const R molar = (lam * R(2.0 / 3.0)) * R(2.016) + (lam * R(1.0 / 3.0)) * R(32.0) +
                     (R(1) - lam) * R(18.016);
-    t = np_max((p * molar) / (rho2 * R(8314.46)), R(kFloor));
-    return d.a * texp(-d.ea / (R(8.314) * t));
+    t = floored(qd(p * molar, rho * R(8314.46)));
+    return d.a * texp(qd(-d.ea, R(8.314) * t));
   }
-  t = np_max(p / rho, R(kFloor));
-  return d.a * texp(-d.ea / t);
+  t = floored(qd(p, rho));
+  return d.a * texp(qd(-d.ea, t));
 }
 
 // One cell: returns false when the reference would reject the input
@@ -1476,19 +1486,19 @@ __device__ __forceinline__ bool react_cell(const Chem<R>& d, R* u, R& lam, R& be
   if (DIM > 1) {     // 2D/3D: move the transverse kinetic energy out of E
     R st = u[2] * u[2];
     if (DIM == 3) st = st + u[3] * u[3];
-    s2 = u[NV - 1] - (R(0.5) * st) / u[0];
+    s2 = u[NV - 1] - qd(hf(st), u[0]);
   }
-  bool ok = finite_(lam) && lam >= R(0) && lam <= R(1);
-  const R e1 = s2 - (R(0.5) * (s1 * s1)) / s0;
-  ok = ok && finite_(s0) && finite_(s1) && finite_(s2) && s0 > R(kFloor) && e1 > R(kFloor);
+  bool ok = finite_(lam) & ge0(lam) & !gt_pos(lam, R(1));
+  const R e1 = s2 - qd(hf(s1 * s1), s0);
+  ok = ok & finite_(s0) & finite_(s1) & finite_(s2) & gt_pos(s0, R(kFloor)) & gt_pos(e1, R(kFloor));
   const R beta_n = znd ? beta : R(1);
-  if (znd) ok = ok && finite_(beta) && beta >= R(0) && beta <= R(1);
+  if (znd) ok = ok & finite_(beta) & ge0(beta) & !gt_pos(beta, R(1));
   const R q = d.q;
   const R lam_n = lam;
   auto advance = [&](R rate, R duration, R& lam_out, R& beta_out) {
     if (znd) {
       const R floor_rate = Exact<R>::value ? R(1e-300) : R(1e-30);
-      const R active = np_max(R(0), duration - beta_n / np_max(rate, floor_rate));
+      const R active = np_max(R(0), duration - qd(beta_n, np_max(rate, floor_rate)));
       lam_out = lam_n * texp((R(-5.0) * rate) * active);
       beta_out = np_min(np_max(beta_n - rate * duration, R(0)), R(1));
     } else {
@@ -1595,7 +1605,7 @@ __global__ void __launch_bounds__(256) react_kernel(StepArgs A, int stage) {
         R w[DIM];
         wave_speeds<R, DIM>(u, gc, w);
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) wmax[k] = fmax(wmax[k], w[k]);
+        for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
       }
     }
     fl = block_or(fl, reinterpret_cast<int*>(red));
@@ -1682,18 +1692,18 @@ __global__ void __launch_bounds__(256) species_kernel(StepArgs A) {
             const R Flo = mf[dd][lo], Fhi = mf[dd][hi];
             const R qlo_l = fetch_scalar<R, DIM>(d, g, q, a - ia, b - ib, p - ip);
             const R qhi_r = fetch_scalar<R, DIM>(d, g, q, a + ia, b + ib, p + ip);
-            const R Glo = Flo * (Flo >= R(0) ? qlo_l : qc);
-            const R Ghi = Fhi * (Fhi >= R(0) ? qc : qhi_r);
+            const R Glo = Flo * (ge0(Flo) ? qlo_l : qc);
+            const R Ghi = Fhi * (ge0(Fhi) ? qc : qhi_r);
             rhoq = rhoq - cu[dd] * (Ghi - Glo);
           }
           R frac;
           if (DIM == 3) {
             // the reference's interval check; FP32 roundoff needs a wider margin
             const R tol = Exact<R>::value ? R(1e-10) : R(1e-5);
-            frac = rhoq / Unew[off];
-            if (frac < -tol || frac > R(1) + tol) fl |= kFlagSpecies;
+            frac = qd(rhoq, Unew[off]);
+            if (lt_(frac, -tol) || gt_pos(frac, R(1) + tol)) fl |= kFlagSpecies;
           } else {
-            frac = rhoq / np_max(Unew[off], R(kFloor));
+            frac = qd(rhoq, floored(Unew[off]));
           }
           qn[off] = np_min(np_max(frac, R(0)), R(1));
         }
@@ -1789,13 +1799,13 @@ __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(StepArgs A, 
   if (j < kGroups * NV) {
     const int k = j % NV, g = j / NV;
     const int m = t1 - t0;
-    for (int r = g; r < m; r += kGroups) v = k < 3 ? fmax(v, vals[k][r]) : v + vals[k][r];
+    for (int r = g; r < m; r += kGroups) v = k < 3 ? soft_fmax_run(v, vals[k][r]) : v + vals[k][r];
   }
   acc[j] = v;
   __syncthreads();
   if (j < NV) {
     double r = acc[j];
-    for (int g = 1; g < kGroups; ++g) r = j < 3 ? fmax(r, acc[g * NV + j]) : r + acc[g * NV + j];
+    for (int g = 1; g < kGroups; ++g) r = j < 3 ? soft_fmax_run(r, acc[g * NV + j]) : r + acc[g * NV + j];
     sh_v[j] = r;
   }
   if (j == 0) sh_f = fl;
@@ -1824,7 +1834,7 @@ __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(StepArgs A, 
         for (int u = 0; u < 8; ++u) {
           if (q0 + u >= nslices) break;
           if (j == NV) f |= __double_bits_as_int(x[u]);
-          else r = j < 3 ? fmax(r, x[u]) : r + x[u];
+          else r = j < 3 ? soft_fmax_run(r, x[u]) : r + x[u];
         }
       }
       if (j < NV) sh_v[j] = r;
@@ -1853,7 +1863,7 @@ __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(StepArgs A, 
     const double dt = st.dt;
     if (lane < nv) {
       double out = 0.0;
-      for (int k = 0; k < d.dim; ++k) out += dt * d.vol / d.h[k] * sh_s[k * 5 + lane];
+      for (int k = 0; k < d.dim; ++k) out += soft_div(dt * d.vol, d.h[k]) * sh_s[k * 5 + lane];
       st.boundary[lane] += out;
       if (d.reactive) st.source[lane] += d.vol * sh_i[lane];
     }

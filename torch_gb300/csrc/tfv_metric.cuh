@@ -119,9 +119,10 @@ __device__ __forceinline__ void primitive_of(const R* u, R g, R* p) {
 #pragma unroll
   for (int c = 2; c < NV - 1; ++c) s = s + u[c] * u[c];
   p[0] = u[0];
+  const Divisor<R> rho(u[0]);
 #pragma unroll
-  for (int c = 1; c < NV - 1; ++c) p[c] = u[c] / u[0];
-  p[NV - 1] = (g - R(1)) * (u[NV - 1] - (R(0.5) * s) / u[0]);
+  for (int c = 1; c < NV - 1; ++c) p[c] = qd(u[c], rho);
+  p[NV - 1] = (g - R(1)) * (u[NV - 1] - qd(hf(s), rho));
 }
 
 // conservative state of face primitives (torchFiniteVolume.py:25-29)
@@ -133,7 +134,7 @@ __device__ __forceinline__ void conservative_of(const R* p, R g, R* u) {
   u[0] = p[0];
 #pragma unroll
   for (int c = 1; c < NV - 1; ++c) u[c] = p[c] * p[0];
-  u[NV - 1] = p[NV - 1] / (g - R(1)) + (R(0.5) * p[0]) * s;
+  u[NV - 1] = qd(p[NV - 1], g - R(1)) + hf(p[0]) * s;
 }
 
 // A padded cell: primitives, gamma and fractions.
@@ -252,7 +253,16 @@ __device__ __forceinline__ int padded_cell(const MArgs<R>& A, int j, const MIdx&
 // limited (torchFiniteVolume.py:105-126)
 template <typename R>
 __device__ __forceinline__ R metric_limited(R minus, R plus, int lim) {
-  const R r = minus / ((fabs(plus) < R(1e-14)) ? R(1e-14) : plus);
+  const R r = qd(minus, guarded(plus, R(1e-14)));
+  if constexpr (Exact<R>::value) {  // region by region, the same values (limiter_phi)
+    switch (lim) {
+      case 0: return limiter_phi<3, 0>(r) * plus;
+      case 1: return limiter_phi<3, 1>(r) * plus;
+      case 2: return limiter_phi<3, 2>(r) * plus;
+      case 3: return limiter_phi<3, 3>(r) * plus;
+      default: return limiter_phi<3, 4>(r) * plus;
+    }
+  }
   const R pos = np_max(r, R(0));
   R phi;
   if (lim == 0) {
@@ -277,8 +287,8 @@ __device__ __forceinline__ void cell_slope(const MCell<R, NV>& m, const MCell<R,
                                            const MCell<R, NV>& p, int lim, R* s) {
 #pragma unroll
   for (int v = 0; v < NV; ++v) s[v] = metric_limited(c.p[v] - m.p[v], p.p[v] - c.p[v], lim);
-  const bool bad = (c.p[0] - R(0.5) * fabs(s[0])) <= R(1e-12) ||
-                   (c.p[NV - 1] - R(0.5) * fabs(s[NV - 1])) <= R(1e-12);
+  const bool bad = le_(c.p[0] - hf(R(fabs(s[0]))), R(1e-12)) ||
+                   le_(c.p[NV - 1] - hf(R(fabs(s[NV - 1]))), R(1e-12));
   if (bad) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) s[v] = s[v] * R(0);
@@ -308,7 +318,7 @@ __global__ void __launch_bounds__(kMThreads) metric_prim_kernel(MArgs<R> A) {
 #pragma unroll
     for (int v = 0; v < NV; ++v) A.P[v * A.nc + off] = p[v];
     if (A.reactive) A.G[off] = g;
-    A.S[off] = sqrt((g * p[NV - 1]) / p[0]);  // as cell_speed forms it
+    A.S[off] = rt(qd(g * p[NV - 1], p[0]));  // as cell_speed forms it
     R s[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) s[v] = R(0);
@@ -316,16 +326,16 @@ __global__ void __launch_bounds__(kMThreads) metric_prim_kernel(MArgs<R> A) {
       const MIdx c = cell_of(off, A);
       const R vol = volume<R, DIM>(A, c);
       const R rho = p[0], pr = p[NV - 1];
-      const R radial = (area<R, DIM>(A, 0, c.i + 1, c) - area<R, DIM>(A, 0, c.i, c)) / vol;
+      const R radial = qd(area<R, DIM>(A, 0, c.i + 1, c) - area<R, DIM>(A, 0, c.i, c), vol);
       s[1] = pr * radial;
       if (A.geometry == kGeoSpherical) {
-        const R invr = radial / R(2);
+        const R invr = hf(radial);
         R sq = R(0);
         if (DIM >= 2) sq = p[2] * p[2];
         if (DIM == 3) sq = sq + p[3] * p[3];
         s[1] = s[1] + (rho * sq) * invr;
         if (DIM >= 2) {
-          const R cot = (area<R, DIM>(A, 1, c.j + 1, c) - area<R, DIM>(A, 1, c.j, c)) / vol;
+          const R cot = qd(area<R, DIM>(A, 1, c.j + 1, c) - area<R, DIM>(A, 1, c.j, c), vol);
           s[2] = pr * cot - ((rho * p[1]) * p[2]) * invr;
           if (DIM == 3) {
             s[2] = s[2] + (rho * (p[3] * p[3])) * cot;
@@ -394,8 +404,8 @@ __device__ __forceinline__ void face_flux(const MArgs<R>& A, int f, const MIdx& 
   R left[NV], right[NV];
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    left[v] = cl.p[v] + R(0.5) * sl[v];
-    right[v] = cr.p[v] - R(0.5) * sr[v];
+    left[v] = cl.p[v] + hf(sl[v]);
+    right[v] = cr.p[v] - hf(sr[v]);
   }
   R gl = cl.g, gr = cr.g;
   // walls mirror the interior face state (torchFiniteVolume.py:164-181)
@@ -425,20 +435,20 @@ __device__ __forceinline__ void face_flux(const MArgs<R>& A, int f, const MIdx& 
   fr[d + 1] = fr[d + 1] + right[NV - 1];
   fl[NV - 1] = fl[NV - 1] + vl * left[NV - 1];
   fr[NV - 1] = fr[NV - 1] + vr * right[NV - 1];
-  const R speed = np_max(fabs(vl) + sqrt((gl * left[NV - 1]) / left[0]),
-                         fabs(vr) + sqrt((gr * right[NV - 1]) / right[0]));
+  const R speed = np_max(fabs(vl) + rt(qd(gl * left[NV - 1], left[0])),
+                         fabs(vr) + rt(qd(gr * right[NV - 1], right[0])));
   const R ar = area<R, DIM>(A, d, f, c);
   R flux0 = R(0);
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    const R flux = ((fl[v] + fr[v]) - (ur[v] - ul[v]) * speed) * R(0.5);
+    const R flux = hf((fl[v] + fr[v]) - (ur[v] - ul[v]) * speed);
     if (v == 0) flux0 = flux;
     W[v] = flux * ar;
   }
   // first-order upwind transport of the fractions (torchFiniteVolume.py:223-226)
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
-    const R up = flux0 >= R(0) ? cl.q[q] : cr.q[q];
+    const R up = ge0(flux0) ? cl.q[q] : cr.q[q];
     T[q] = q < A.nfrac ? (flux0 * up) * ar : R(0);
   }
 }
@@ -649,7 +659,7 @@ __global__ void __launch_bounds__(kMThreads) metric_update_kernel(MArgs<R> A, in
   for (int64_t off = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; off < A.nc;
        off += (int64_t)gridDim.x * blockDim.x) {
     const MIdx c = cell_of(off, A);
-    const R vol = volume<R, DIM>(A, c);
+    const Divisor<R> vol(volume<R, DIM>(A, c));
     R k[NV], kq[2] = {R(0), R(0)};
 #pragma unroll
     for (int v = 0; v < NV; ++v) k[v] = ro(&A.K[v * A.nc + off]);
@@ -659,10 +669,10 @@ __global__ void __launch_bounds__(kMThreads) metric_update_kernel(MArgs<R> A, in
       const int64_t lo = face_off(d, cc[d], c, A.n), hi = face_off(d, cc[d] + 1, c, A.n);
       const int64_t nf = A.nf[d];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) k[v] = k[v] - (ro(&A.W[d][v * nf + hi]) - ro(&A.W[d][v * nf + lo])) / vol;
+      for (int v = 0; v < NV; ++v) k[v] = k[v] - qd(ro(&A.W[d][v * nf + hi]) - ro(&A.W[d][v * nf + lo]), vol);
 #pragma unroll
       for (int q = 0; q < 2; ++q) if (q < A.nfrac)
-        kq[q] = kq[q] - (ro(&A.T[d][q * nf + hi]) - ro(&A.T[d][q * nf + lo])) / vol;
+        kq[q] = kq[q] - qd(ro(&A.T[d][q * nf + hi]) - ro(&A.T[d][q * nf + lo]), vol);
     }
     R out[NV], oq[2];
     if (stage == 1) {
@@ -671,15 +681,15 @@ __global__ void __launch_bounds__(kMThreads) metric_update_kernel(MArgs<R> A, in
       const R rho0 = ro(&A.U[off]);
 #pragma unroll
       for (int q = 0; q < 2; ++q) if (q < A.nfrac)
-        oq[q] = (rho0 * ro(&A.Q[q][off]) + dt * kq[q]) / out[0];
+        oq[q] = qd(rho0 * ro(&A.Q[q][off]) + dt * kq[q], out[0]);
     } else {
 #pragma unroll
       for (int v = 0; v < NV; ++v)
-        out[v] = R(0.5) * ((ro(&A.U0[v * A.nc + off]) + ro(&A.Us[v * A.nc + off])) + dt * k[v]);
+        out[v] = hf((ro(&A.U0[v * A.nc + off]) + ro(&A.Us[v * A.nc + off])) + dt * k[v]);
       const R rho0 = ro(&A.U0[off]), rhos = ro(&A.Us[off]);
 #pragma unroll
       for (int q = 0; q < 2; ++q) if (q < A.nfrac)
-        oq[q] = (R(0.5) * ((rho0 * ro(&A.Q0[q][off]) + rhos * ro(&A.Qs[q][off])) + dt * kq[q])) / out[0];
+        oq[q] = qd(hf((rho0 * ro(&A.Q0[q][off]) + rhos * ro(&A.Qs[q][off])) + dt * kq[q]), out[0]);
     }
     if (!physical_cell<R, NV>(out)) err |= kMErrNonphysical;
     // the reference's interval check (1e-12); single-precision roundoff of a
@@ -687,7 +697,7 @@ __global__ void __launch_bounds__(kMThreads) metric_update_kernel(MArgs<R> A, in
     const R tol = Exact<R>::value ? R(1e-12) : R(1e-5);
 #pragma unroll
     for (int q = 0; q < 2; ++q) if (q < A.nfrac) {
-      if (oq[q] < -tol || oq[q] > R(1) + tol) err |= kMErrFraction;
+      if (lt_(oq[q], -tol) || gt_pos(oq[q], R(1) + tol)) err |= kMErrFraction;
       oq[q] = np_min(np_max(oq[q], R(0)), R(1));  // np.clip
       A.Qout[q][off] = oq[q];
     }
@@ -921,19 +931,19 @@ __device__ __forceinline__ R direction_rate(const MArgs<R>& A, const MIdx& c, in
   MCell<R, NV> o;
   if (cd == 0) {  // boundary_state of the low face
     err |= padded_cell<R, NV, D>(A, 0, c, o);
-    fs_lo = np_max(s, fabs(o.p[D + 1]) + sqrt((o.g * o.p[NV - 1]) / o.p[0]));
+    fs_lo = np_max(s, fabs(o.p[D + 1]) + rt(qd(o.g * o.p[NV - 1], o.p[0])));
   } else {  // interior neighbour below
     const int64_t nb = off - stride;
     fs_lo = np_max(fabs(ro(&A.P[(D + 1) * A.nc + nb])) + ro(&A.S[nb]), s);
   }
   if (cd == n - 1) {
     err |= padded_cell<R, NV, D>(A, n + 1, c, o);
-    fs_hi = np_max(s, fabs(o.p[D + 1]) + sqrt((o.g * o.p[NV - 1]) / o.p[0]));
+    fs_hi = np_max(s, fabs(o.p[D + 1]) + rt(qd(o.g * o.p[NV - 1], o.p[0])));
   } else {  // interior neighbour above
     const int64_t nb = off + stride;
     fs_hi = np_max(s, fabs(ro(&A.P[(D + 1) * A.nc + nb])) + ro(&A.S[nb]));
   }
-  return np_max(area<R, DIM>(A, D, cd, c) * fs_lo, area<R, DIM>(A, D, cd + 1, c) * fs_hi) / vol;
+  return qd(np_max(area<R, DIM>(A, D, cd, c) * fs_lo, area<R, DIM>(A, D, cd + 1, c) * fs_hi), vol);
 }
 
 template <typename R, int DIM>
@@ -951,7 +961,7 @@ __global__ void __launch_bounds__(kMThreads) metric_rate_kernel(MArgs<R> A) {
     R rate = direction_rate<R, DIM, 0>(A, c, off, self, vol, err);
     if constexpr (DIM >= 2) rate = rate + direction_rate<R, DIM, 1>(A, c, off, self, vol, err);
     if constexpr (DIM == 3) rate = rate + direction_rate<R, DIM, 2>(A, c, off, self, vol, err);
-    if (!(rate == rate) || isinf(rate)) err |= kMErrRate;
+    if (!finite_(rate)) err |= kMErrRate;
     best = np_max(best, rate);
   }
   const R top = block_max(best, red);
@@ -1073,10 +1083,10 @@ __global__ void __launch_bounds__(kMThreads) rusanov_faces_kernel(
       }
     fl[NV - 1] = fl[NV - 1] + vl * left[NV - 1];
     fr[NV - 1] = fr[NV - 1] + vr * right[NV - 1];
-    const R speed = np_max(fabs(vl) + sqrt((gl * left[NV - 1]) / left[0]),
-                           fabs(vr) + sqrt((gr * right[NV - 1]) / right[0]));
+    const R speed = np_max(fabs(vl) + rt(qd(gl * left[NV - 1], left[0])),
+                           fabs(vr) + rt(qd(gr * right[NV - 1], right[0])));
 #pragma unroll
-    for (int v = 0; v < NV; ++v) out[v * n + i] = R(0.5) * ((fl[v] + fr[v]) - speed * (ur[v] - ul[v]));
+    for (int v = 0; v < NV; ++v) out[v * n + i] = hf((fl[v] + fr[v]) - speed * (ur[v] - ul[v]));
   }
 }
 

@@ -16,6 +16,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tfv_soft64.cuh"
+
 namespace tfv {
 
 constexpr double kFloor = 1e-12;  // density / pressure floor
@@ -31,8 +33,9 @@ struct Exact<double> {
 };
 
 // numpy.maximum / numpy.minimum: NaN propagates, first operand wins ties.
-__device__ __forceinline__ double np_max(double a, double b) { return (a >= b || a != a) ? a : b; }
-__device__ __forceinline__ double np_min(double a, double b) { return (a <= b || a != a) ? a : b; }
+// Double precision: integer comparisons (tfv_soft64.cuh), not the FP64 pipe.
+__device__ __forceinline__ double np_max(double a, double b) { return soft_max(a, b); }
+__device__ __forceinline__ double np_min(double a, double b) { return soft_min(a, b); }
 __device__ __forceinline__ float np_max(float a, float b) {
   float r;
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
@@ -52,17 +55,67 @@ __device__ __forceinline__ float np_max3(float a, float b, float c) {
   return r;
 }
 
-// a / b: IEEE division (double) or the approximate single-precision one.
-__device__ __forceinline__ double dv(double a, double b) { return a / b; }
+// a / b: IEEE division (double, on the integer pipe) or the approximate
+// single-precision one.
+__device__ __forceinline__ double dv(double a, double b) { return soft_div(a, b); }
 __device__ __forceinline__ float dv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float rcp(float b) { return __fdividef(1.0f, b); }
-
-// np.where(abs(x) < g, g, x)
+// a / b as the operator: IEEE (double), the unit's division flags (float).
+__device__ __forceinline__ double qd(double a, double b) { return soft_div(a, b); }
+__device__ __forceinline__ float qd(float a, float b) { return a / b; }
+// a divisor used several times (double: its reciprocal estimate formed once)
 template <typename R>
-__device__ __forceinline__ R guarded(R x, R g) { return (fabs(x) < g) ? g : x; }
-
+struct Divisor {
+  R b;
+  __device__ __forceinline__ explicit Divisor(R b_) : b(b_) {}
+};
+template <>
+struct Divisor<double> {
+  SoftDivisor d;
+  __device__ __forceinline__ explicit Divisor(double b) : d(soft_divisor(b)) {}
+};
+__device__ __forceinline__ double qd(double a, const Divisor<double>& d) { return soft_div(a, d.d); }
+__device__ __forceinline__ float qd(float a, const Divisor<float>& d) { return a / d.b; }
+__device__ __forceinline__ double rt(double x) { return soft_sqrt(x); }
+__device__ __forceinline__ float rt(float x) { return sqrtf(x); }
+// x / 2 and 2 x, exact
+__device__ __forceinline__ double hf(double x) { return soft_half(x); }
+__device__ __forceinline__ float hf(float x) { return 0.5f * x; }
+__device__ __forceinline__ double tw(double x) { return soft_twice(x); }
+__device__ __forceinline__ float tw(float x) { return 2.0f * x; }
+// comparisons (false for NaN)
+__device__ __forceinline__ bool lt_(double a, double b) { return soft_lt(a, b); }
+__device__ __forceinline__ bool lt_(float a, float b) { return a < b; }
+__device__ __forceinline__ bool le_(double a, double b) { return soft_le(a, b); }
+__device__ __forceinline__ bool le_(float a, float b) { return a <= b; }
+__device__ __forceinline__ bool le0(double x) { return soft_le0(x); }
+__device__ __forceinline__ bool le0(float x) { return x <= 0.0f; }
+__device__ __forceinline__ bool ge0(double x) { return soft_ge0(x); }
+__device__ __forceinline__ bool ge0(float x) { return x >= 0.0f; }
+__device__ __forceinline__ bool gt0(double x) { return soft_gt0(x); }
+__device__ __forceinline__ bool gt0(float x) { return x > 0.0f; }
+__device__ __forceinline__ bool lt0(double x) { return soft_lt0(x); }
+__device__ __forceinline__ bool lt0(float x) { return x < 0.0f; }
+// x > c and |x| < c for a positive compile-time constant c
+__device__ __forceinline__ bool gt_pos(double x, double c) { return soft_gt_pos(x, c); }
+__device__ __forceinline__ bool gt_pos(float x, float c) { return x > c; }
+__device__ __forceinline__ bool abs_lt(double x, double c) { return soft_abs_lt(x, c); }
+__device__ __forceinline__ bool abs_lt(float x, float c) { return fabsf(x) < c; }
+// np_max(x, c) for a positive compile-time constant c
+__device__ __forceinline__ double max_pos(double x, double c) { return soft_max_pos(x, c); }
+__device__ __forceinline__ float max_pos(float x, float c) { return np_max(x, c); }
 template <typename R>
-__device__ __forceinline__ bool finite_(R x) { return isfinite(x); }
+__device__ __forceinline__ R floored(R x) { return max_pos(x, R(kFloor)); }
+// fmax(m, x) of a running maximum m >= 0
+__device__ __forceinline__ double run_max(double m, double x) { return soft_fmax_run(m, x); }
+__device__ __forceinline__ float run_max(float m, float x) { return fmaxf(m, x); }
+
+// np.where(abs(x) < g, g, x), g a positive compile-time constant
+template <typename R>
+__device__ __forceinline__ R guarded(R x, R g) { return abs_lt(x, g) ? g : x; }
+
+__device__ __forceinline__ bool finite_(double x) { return soft_isfinite(x); }
+__device__ __forceinline__ bool finite_(float x) { return isfinite(x); }
 
 // Constant gamma of an instance descriptor in the arithmetic type: single
 // precision reads its float copy instead of converting the double per cell
@@ -78,6 +131,41 @@ __device__ __forceinline__ float desc_gamma(const D& d, float) { return d.gamma_
 // 2D: python/cfdSolver/torchSolver2D.py:124-168 (VanLeer/Albada zero for
 //     r <= 0, Unos without the (1+2r)/3 bound).
 // --------------------------------------------------------------------------
+// phi(r) in double precision, region by region: the numpy.maximum /
+// numpy.minimum nests of the reference reduce to comparisons of r with
+// constants whose low word is zero, decided by r's high word, and each region
+// returns the nest's value bit for bit (zeros with their sign, NaN for NaN).
+template <int DIM, int LIM>
+__device__ __forceinline__ double limiter_phi(double r) {
+  const uint32_t h = s64_hi(r), l = s64_lo(r);
+  const bool nan = soft_isnan(r);
+  const bool zero = ((h << 1) | l) == 0u;
+  const bool pos = (int32_t)h >= 0 && !zero;  // r > 0 (NaN apart)
+  double phi;
+  if (LIM == 0) {  // VanLeer: 2 pos / (1 + pos), pos = max(r, 0)
+    phi = soft_div(soft_twice(r), 1.0 + r);
+    if (!pos) phi = (DIM == 3 && zero) ? r : 0.0;  // max(-0, 0) is -0
+  } else if (LIM == 1) {  // Albada: (pos^2 + pos) / (pos^2 + 1)
+    const double q = r * r;
+    phi = soft_div(q + r, q + 1.0);
+    if (!pos) phi = 0.0;
+  } else if (LIM == 2) {  // MINBEE: max(0, min(r, 1))
+    phi = h < 0x3ff00000u ? r : 1.0;
+    if (!pos) phi = 0.0;
+  } else if (LIM == 3) {  // Superbee: max(0, max(min(2r, 1), min(r, 2)))
+    phi = h < 0x40000000u ? r : 2.0;
+    if (h < 0x3ff00000u) phi = h < 0x3fe00000u ? soft_twice(r) : 1.0;
+    if (!pos) phi = 0.0;
+  } else {  // Unos: max(0, min(min(2, 2r), (2 + r) / 3 [, (1 + 2r) / 3 in 3D]))
+    const double r2 = soft_twice(r);
+    const double m = h >= 0x3ff00000u ? 2.0 : r2;
+    const double a = soft_div(2.0 + r, 3.0);
+    phi = DIM == 3 ? soft_min(soft_min(m, a), soft_div(1.0 + r2, 3.0)) : soft_min(m, a);
+    if (!pos) phi = 0.0;
+  }
+  return nan ? r : phi;
+}
+
 template <typename R, int DIM, int LIM>
 __device__ __forceinline__ R limited_slope(R um, R uc, R up) {
   const R minus = uc - um;
@@ -111,24 +199,16 @@ __device__ __forceinline__ R limited_slope(R um, R uc, R up) {
   }
   const R r = dv(minus, guarded(plus, R(kGuard)));
   R phi;
-  if (LIM == 1) {  // Albada
+  if constexpr (Exact<R>::value) {
+    phi = limiter_phi<DIM, LIM>(r);
+  } else if (LIM == 1) {  // Albada
     const R pos = np_max(r, R(0));
     phi = dv(pos * pos + pos, pos * pos + R(1));
     if (DIM == 2 && !(r > R(0))) phi = R(0);
-  } else if (LIM == 2) {  // MINBEE
-    phi = np_max(R(0), np_min(r, R(1)));
-  } else if (LIM == 3) {  // Superbee
-    phi = np_max(R(0), np_max(np_min(R(2) * r, R(1)), np_min(r, R(2))));
-  } else if (LIM == 4) {  // Unos
-    if (DIM == 3)
-      phi = np_max(R(0), np_min(np_min(np_min(R(2), R(2) * r), dv(R(2) + r, R(3))),
-                                dv(R(1) + R(2) * r, R(3))));
-    else
-      phi = np_max(R(0), np_min(np_min(R(2), R(2) * r), dv(R(2) + r, R(3))));
-  } else {  // VanLeer
-    const R pos = np_max(r, R(0));
-    phi = dv(R(2) * pos, R(1) + pos);
-    if (DIM == 2 && !(r > R(0))) phi = R(0);
+  } else {  // Unos (MINBEE, Superbee and VanLeer returned above)
+    phi = np_min(np_min(R(2), R(2) * r), dv(R(2) + r, R(3)));
+    if (DIM == 3) phi = np_min(phi, dv(R(1) + R(2) * r, R(3)));
+    phi = np_max(R(0), phi);
   }
   return phi * plus;
 }
@@ -145,9 +225,9 @@ __device__ __forceinline__ void flux3(const R* u, R g, int m, R* f) {
   const R ssum = (u[1] * u[1] + u[2] * u[2]) + u[3] * u[3];
   R p, vel;
   if constexpr (Exact<R>::value) {
-    const R rho = u[0];
-    p = (g - R(1)) * (u[4] - (R(0.5) * ssum) / rho);
-    vel = u[m] / rho;
+    const Divisor<R> rho(u[0]);
+    p = (g - R(1)) * (u[4] - qd(hf(ssum), rho));
+    vel = qd(u[m], rho);
   } else {
     const R irho = rcp(u[0]);
     p = (g - R(1)) * (u[4] - R(0.5) * ssum * irho);
@@ -162,17 +242,18 @@ __device__ __forceinline__ void flux3(const R* u, R g, int m, R* f) {
 
 template <typename R>
 __device__ __forceinline__ void flux2(const R* u, R g, int normal, R* f) {
-  const R rho = np_max(u[0], R(kFloor));
+  const R rho = floored(u[0]);
   R vx, vy;
   if constexpr (Exact<R>::value) {
-    vx = u[1] / rho;
-    vy = u[2] / rho;
+    const Divisor<R> dr(rho);
+    vx = qd(u[1], dr);
+    vy = qd(u[2], dr);
   } else {
     const R irho = rcp(rho);
     vx = u[1] * irho;
     vy = u[2] * irho;
   }
-  const R p = np_max((g - R(1)) * (u[3] - (R(0.5) * rho) * (vx * vx + vy * vy)), R(kFloor));
+  const R p = floored((g - R(1)) * (u[3] - hf(rho) * (vx * vx + vy * vy)));
   if (normal == 0) {
     f[0] = rho * vx;
     f[1] = rho * (vx * vx) + p;
@@ -195,8 +276,8 @@ __device__ __forceinline__ bool physical_cell(const R* u) {
   if constexpr (Exact<R>::value) {
     bool ok = true;
 #pragma unroll
-    for (int c = 0; c < NV; ++c) ok = ok && finite_(u[c]);
-    return ok && (u[0] > R(kFloor)) && (u[NV - 1] - (R(0.5) * s) / u[0] > R(kFloor));
+    for (int c = 0; c < NV; ++c) ok = ok & finite_(u[c]);
+    return ok & gt_pos(u[0], R(kFloor)) & gt_pos(u[NV - 1] - qd(hf(s), u[0]), R(kFloor));
   } else {
     // one finiteness test: any NaN or infinity makes the sum non-finite
     R all = u[0];
@@ -214,26 +295,119 @@ __device__ __forceinline__ bool physical_cell(const R* u) {
 // that can be selected is formed; values are identical to evaluating both.
 // Where no wave-speed mask holds (NaN speeds) the result is NaN.
 // --------------------------------------------------------------------------
-template <typename R, int NT>
-__device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* out) {
+// Double precision: only the flux and the star state of the side that the
+// masks select are formed (values identical to evaluating both).
+template <int NT>
+__device__ __forceinline__ void hllc_f64(const double* ul, const double* ur, double gl, double gr,
+                                         double* out) {
+  using R = double;
   constexpr int NV = NT + 3;
   constexpr int E = NV - 1;
-  constexpr bool X = Exact<R>::value;
-  const R g = R(0.5) * (gl + gr);
-  const R rl = np_max(ul[0], R(kFloor));
-  const R rr = np_max(ur[0], R(kFloor));
-  R irl = R(0), irr = R(0);
-  if constexpr (!X) {
-    irl = rcp(rl);
-    irr = rcp(rr);
-  }
-  const R unl = X ? ul[1] / rl : ul[1] * irl;
-  const R unr = X ? ur[1] / rr : ur[1] * irr;
+  const R g = hf(gl + gr);
+  const R rl = floored(ul[0]);
+  const R rr = floored(ur[0]);
+  const Divisor<R> dl(rl), dr(rr);
+  const R unl = qd(ul[1], dl);
+  const R unr = qd(ur[1], dr);
   R utl[NT], utr[NT];
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    utl[t] = X ? ul[2 + t] / rl : ul[2 + t] * irl;
-    utr[t] = X ? ur[2 + t] / rr : ur[2 + t] * irr;
+    utl[t] = qd(ul[2 + t], dl);
+    utr[t] = qd(ur[2 + t], dr);
+  }
+  R stl = utl[0] * utl[0], str = utr[0] * utr[0];
+#pragma unroll
+  for (int t = 1; t < NT; ++t) {
+    stl = stl + utl[t] * utl[t];
+    str = str + utr[t] * utr[t];
+  }
+  const R kel = hf(rl) * (unl * unl + stl);
+  const R ker = hf(rr) * (unr * unr + str);
+  const R pl = floored((gl - R(1)) * (ul[E] - kel));
+  const R pr = floored((gr - R(1)) * (ur[E] - ker));
+  const R al = rt(qd(gl * pl, dl));
+  const R ar = rt(qd(gr * pr, dr));
+
+  const R sql = rt(rl);
+  const R sqr = rt(rr);
+  const R inv = qd(R(1), sql + sqr);
+  const R uroe = (sql * unl + sqr * unr) * inv;
+  R vsum;
+  {
+    const R v0 = (sql * utl[0] + sqr * utr[0]) * inv;
+    vsum = v0 * v0;
+#pragma unroll
+    for (int t = 1; t < NT; ++t) {
+      const R vt = (sql * utl[t] + sqr * utr[t]) * inv;
+      vsum = vsum + vt * vt;
+    }
+  }
+  const R epl = ul[E] + pl, epr = ur[E] + pr;
+  const R hl = qd(epl, dl);
+  const R hr = qd(epr, dr);
+  const R hroe = (sql * hl + sqr * hr) * inv;
+  const R keroe = hf(uroe * uroe + vsum);
+  const R aroe = rt(floored((g - R(1)) * (hroe - keroe)));
+
+  const R sL = np_min(unl - al, uroe - aroe);
+  const R sR = np_max(unr + ar, uroe + aroe);
+  const R den = guarded(rl * (sL - unl) - rr * (sR - unr), R(kGuard));
+  const R ss = dv(((pr - pl) + (rl * unl) * (sL - unl)) - (rr * unr) * (sR - unr), den);
+
+  const bool mr = le0(sR);
+  const bool ssn = le0(ss);
+  const bool mstar = (ssn && ge0(sR)) || (le0(sL) && ge0(ss));
+  const bool ml = ge0(sL);
+  // the side whose flux the selected region reads (right supersonic, then the
+  // star region of the side ss picks, then left supersonic)
+  const bool right = mr || (mstar && ssn);
+  const R rho = right ? rr : rl;
+  const R un = right ? unr : unl;
+  const R p = right ? pr : pl;
+  const R s = right ? sR : sL;
+  const R uE = right ? ur[E] : ul[E];
+  R f[NV];
+  f[0] = rho * un;
+  f[1] = rho * (un * un) + p;
+#pragma unroll
+  for (int t = 0; t < NT; ++t) f[2 + t] = (rho * un) * (right ? utr[t] : utl[t]);
+  f[E] = un * (right ? epr : epl);
+  const R gap = s - ss;
+  if (!mr && mstar && !abs_lt(gap, R(kFloor))) {  // star state of that side
+    const R dss = guarded(gap, R(kGuard));
+    const R rho_s = floored(rho * dv(s - un, dss));
+    const R dun = guarded(s - un, R(kGuard));
+    R star[NV];
+    star[0] = rho_s;
+    star[1] = rho_s * ss;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) star[2 + t] = rho_s * (right ? utr[t] : utl[t]);
+    star[E] = rho_s * (qd(uE, right ? dr : dl) + (ss - un) * (ss + qd(p, rho * dun)));
+#pragma unroll
+    for (int c = 0; c < NV; ++c) f[c] = f[c] + s * (star[c] - (right ? ur[c] : ul[c]));
+  }
+#pragma unroll
+  for (int c = 0; c < NV; ++c) out[c] = (mr || mstar || ml) ? f[c] : R(NAN);
+}
+
+// Single precision: both physical fluxes (measured faster in 2D).
+template <int NT>
+__device__ __forceinline__ void hllc_f32(const float* ul, const float* ur, float gl, float gr,
+                                         float* out) {
+  using R = float;
+  constexpr int NV = NT + 3;
+  constexpr int E = NV - 1;
+  const R g = R(0.5) * (gl + gr);
+  const R rl = np_max(ul[0], R(kFloor));
+  const R rr = np_max(ur[0], R(kFloor));
+  const R irl = rcp(rl), irr = rcp(rr);
+  const R unl = ul[1] * irl;
+  const R unr = ur[1] * irr;
+  R utl[NT], utr[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) {
+    utl[t] = ul[2 + t] * irl;
+    utr[t] = ur[2 + t] * irr;
   }
   R stl = utl[0] * utl[0], str = utr[0] * utr[0];
 #pragma unroll
@@ -245,8 +419,8 @@ __device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* ou
   const R ker = (R(0.5) * rr) * (unr * unr + str);
   const R pl = np_max((gl - R(1)) * (ul[E] - kel), R(kFloor));
   const R pr = np_max((gr - R(1)) * (ur[E] - ker), R(kFloor));
-  const R al = X ? sqrt((gl * pl) / rl) : sqrt(gl * pl * irl);
-  const R ar = X ? sqrt((gr * pr) / rr) : sqrt(gr * pr * irr);
+  const R al = sqrt(gl * pl * irl);
+  const R ar = sqrt(gr * pr * irr);
 
   R fl[NV], fr[NV];
   fl[0] = rl * unl;
@@ -263,7 +437,7 @@ __device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* ou
 
   const R sql = sqrt(rl);
   const R sqr = sqrt(rr);
-  const R inv = X ? R(1) / (sql + sqr) : rcp(sql + sqr);
+  const R inv = rcp(sql + sqr);
   const R uroe = (sql * unl + sqr * unr) * inv;
   R vsum;
   {
@@ -275,8 +449,8 @@ __device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* ou
       vsum = vsum + vt * vt;
     }
   }
-  const R hl = X ? (ul[E] + pl) / rl : (ul[E] + pl) * irl;
-  const R hr = X ? (ur[E] + pr) / rr : (ur[E] + pr) * irr;
+  const R hl = (ul[E] + pl) * irl;
+  const R hr = (ur[E] + pr) * irr;
   const R hroe = (sql * hl + sqr * hr) * inv;
   const R keroe = R(0.5) * (uroe * uroe + vsum);
   const R aroe = sqrt(np_max((g - R(1)) * (hroe - keroe), R(kFloor)));
@@ -301,11 +475,7 @@ __device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* ou
   star[1] = rho_s * ss;
 #pragma unroll
   for (int t = 0; t < NT; ++t) star[2 + t] = rho_s * (right ? utr[t] : utl[t]);
-  if constexpr (X) {
-    star[E] = rho_s * (uE / rho + (ss - un) * (ss + p / (rho * dun)));
-  } else {
-    star[E] = rho_s * (uE * (right ? irr : irl) + (ss - un) * (ss + dv(p, rho * dun)));
-  }
+  star[E] = rho_s * (uE * (right ? irr : irl) + (ss - un) * (ss + dv(p, rho * dun)));
   const bool close = fabs(s - ss) < R(kFloor);
 
   const bool mr = (R(0) >= sR);
@@ -323,6 +493,14 @@ __device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* ou
     if (mr) v = fr[c];
     out[c] = v;
   }
+}
+
+template <typename R, int NT>
+__device__ __forceinline__ void hllc(const R* ul, const R* ur, R gl, R gr, R* out) {
+  if constexpr (Exact<R>::value)
+    hllc_f64<NT>(ul, ur, gl, gr, out);
+  else
+    hllc_f32<NT>(ul, ur, gl, gr, out);
 }
 
 // Rotation into the normal basis (python/cfdSolver/torchFlux.py:36-39):
