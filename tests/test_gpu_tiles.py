@@ -75,3 +75,24 @@ def test_1d_default_tiling_equals_whole_warp_tiles(n, precision):
             states.append((sim.state, sim.time))
         np.testing.assert_array_equal(states[0][0], states[1][0])
         assert states[0][1] == states[1][1]
+
+
+@pytest.mark.parametrize("counts,tile,precision", [
+    ((132, 9), (124, 1, 32), "fp32"), ((4, 3), (128, 1, 4), "fp32"),
+    ((20, 17, 9), (16, 16, 40), "fp32"), ((16, 16, 16), (16, 16, 5), "fp32"),
+    ((4, 2, 3), (32, 8, 16), "fp32"), ((34, 11), (32, 1, 4), "fp64"),
+    ((18, 5, 6), (32, 4, 32), "fp64"),
+])
+@pytest.mark.parametrize("boundary", ["Open", "Reflective", "Periodic"])
+def test_element_copies_stage_what_tensor_copies_stage(counts, tile, precision, boundary):
+    """Grids whose rows allow tensor copies, staged by tensor copies and by one
+    asynchronous copy per cell (what rows of other lengths take)."""
+    states = []
+    for tma in (1, 0):
+        sim = torch_gb300.Simulation(rough(counts), [1.0] * len(counts), t_end=1.0,
+                                     limiter="MINBEE", boundaries=[boundary] * len(counts),
+                                     precision=precision, tile=tile + (0, tma))
+        for _ in range(3):
+            sim.step()
+        states.append(sim.state)
+    np.testing.assert_array_equal(states[0], states[1])
