@@ -260,6 +260,7 @@ template <typename R, bool VARG>
 // otherwise (bind, re-plan, integrals) the integrals of the state are written.
 __global__ void __launch_bounds__(256) waves1d_kernel(StepArgs A, int in_step) {
   __shared__ double red[40];
+  pdl_wait();
   if (in_step == 2) {  // usually no instance took the fallback
     int any = 0;
     for (int k = threadIdx.x; k < A.ninst; k += blockDim.x)
@@ -394,6 +395,7 @@ __device__ __forceinline__ void recon1(const InstDesc& d, const InstState& st, c
 // (python/cfdSolver/torchSolver.py:412-491).
 template <typename R, bool VARG>
 __global__ void __launch_bounds__(256) recon1d_kernel(StepArgs A) {
+  pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
     if (!TFV_IN(45, t, A.ntiles)) continue;
     const Tile T = A.tiles[t];
@@ -456,6 +458,7 @@ __device__ __forceinline__ void face_flux1(const InstDesc& d, const R* U, const 
 template <typename R, bool VARG>
 __global__ void __launch_bounds__(256) update1d_kernel(StepArgs A, int first_order) {
   __shared__ double red[40];
+  pdl_wait();
   if (first_order) {  // the fallback pass: usually no instance is flagged
     int any = 0;
     for (int k = threadIdx.x; k < A.ninst; k += blockDim.x)
@@ -582,6 +585,7 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
   R* fx = rc + 6 * W;                          // [3][W] flux at the face left of slot k
   R* un_s = fx + 3 * W;                        // [3][tx + 2] new state of the targets
   const int TS = A.tx + 2;
+  pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
     if (!TFV_IN(45, t, A.ntiles)) continue;
     const Tile T = A.tiles[t];

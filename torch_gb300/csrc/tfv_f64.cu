@@ -22,7 +22,6 @@ namespace tfv {
 cudaError_t launch_finalize(const StepArgs& A, int mode, int fp32, double* integrals_out,
                             cudaStream_t s) {
   const dim3 grid(A.fin_slices > 0 ? A.fin_slices : 1, A.ninst);
-  finalize_kernel<<<grid, kFinalizeThreads, 0, s>>>(A, mode, fp32, integrals_out);
-  return cudaGetLastError();
+  return launch_pdl(finalize_kernel, grid, kFinalizeThreads, 0, s, A, mode, fp32, integrals_out);
 }
 }  // namespace tfv

@@ -35,6 +35,18 @@ enum : int { kBcOpen = 0, kBcReflective = 1, kBcPeriodic = 2, kBcInflow = 3 };
 constexpr int kFinalizeThreads = 256;  // threads of a finalize CTA
 constexpr int kPartVals = 23;          // partials per tile: 3 maxima, 15 boundary sums, 5 integrals
 
+// Programmatic dependent launch: the kernels of a step are launched so that
+// the next one is set up as its predecessor completes, and every kernel waits
+// here for that completion (and the visibility of its writes) before it reads
+// or writes anything that another kernel touches, on every path: a kernel that
+// exited without waiting would release its successor too early.  No kernel
+// triggers its successor earlier: CTAs that wait on an SM spoil the placement
+// of the running ones (2D 256^2 FP64, 16 steps: 2.03 ms with this wait alone,
+// 2.13 with triggers, 2.15 with plain launches; 1000-cell FP64 tube step 64 /
+// 64 / 75 us; 16 FP32 tubes, 64 steps 2.10 / 2.12 / 2.14 ms).  A no-op where
+// the launch did not ask for it.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // an int carried in a double slot of the finalize records (bit copy)
 __device__ __forceinline__ double __int_as_double_bits(int v) {
   return __longlong_as_double((long long)(unsigned)v);
@@ -1086,6 +1098,7 @@ __global__ void __launch_bounds__(256, TFV_HYDRO_MIN_BLOCKS) hydro_kernel(StepAr
     fence_mbar_init();
   }
   __syncthreads();
+  pdl_wait();
   uint32_t bar_phase = 0;  // parity of the next completion of each slot's barrier
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x)
     if (!hydro_tile<R, DIM, VARG, LIM>(A, t, smem, S, bar_phase)) break;
@@ -1149,6 +1162,7 @@ template <typename R, int DIM, bool VARG>
 __global__ void __launch_bounds__(256) fallback_kernel(StepArgs A) {
   constexpr int NV = DIM + 2;
   __shared__ double red[40];
+  pdl_wait();
   {
     // usually no instance is flagged: one look at the instance states instead
     // of walking the tile table
@@ -1284,6 +1298,7 @@ template <typename R, int DIM, bool VARG>
 __global__ void __launch_bounds__(256) waves_kernel(StepArgs A, int sums) {
   constexpr int NV = DIM + 2;
   __shared__ double red[40];
+  pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
     if (!TFV_IN(30, t, A.ntiles)) continue;
     const Tile T = A.tiles[t];
@@ -1397,65 +1412,79 @@ __device__ __forceinline__ void set_dt(const InstDesc& d, InstState& st, double 
   }
 }
 
-__device__ __forceinline__ void plan_next(const InstDesc& d, InstState& st, const double* w,
-                                          int fp32) {
-  if (st.time == d.t_end) {
-    st.status = kDone;
-    return;
-  }
-  if (st.steps >= d.max_steps) {
-    st.status = kErrMaxSteps;
-    return;
-  }
-  double dt = cfl_dt(d, w);
-  if (fp32) dt = (double)(float)dt;
-  const double rem = d.t_end - st.time;
-  if (rem < dt) dt = rem;
-  set_dt(d, st, dt);
-  if (!isfinite(dt) || dt <= 0.0 || st.time + dt == st.time) {
-    st.status = kErrStall;
-    return;
-  }
-  st.status = kReady;
+// What the commit and the plan of an instance read, loaded by every lane of
+// warp 0 as the finalize kernel starts, beside the tile records: read where
+// they are used, each was a round trip to L2 on the kernel's critical path.
+struct FinPre {
+  double time, dt, boundary, source;  // boundary, source: this lane's component
+  double h, vol, cfl, t_end;          // h: spacing of this lane's direction (lane mod 3)
+  int64_t steps, max_steps;
+  int32_t cur, status, fb_word, fallback_steps;
+};
+__device__ __forceinline__ FinPre fin_load(const InstDesc& d, const InstState& st, int lane) {
+  FinPre p;
+  p.time = st.time;
+  p.dt = st.dt;
+  p.boundary = lane < 5 ? st.boundary[lane] : 0.0;
+  p.source = lane < 5 ? st.source[lane] : 0.0;
+  p.h = d.h[lane % 3];
+  p.vol = d.vol;
+  p.cfl = d.cfl;
+  p.t_end = d.t_end;
+  p.steps = st.steps;
+  p.max_steps = d.max_steps;
+  p.cur = st.cur;
+  p.status = st.status;
+  p.fb_word = st.fb_word;
+  p.fallback_steps = st.fallback_steps;
+  return p;
 }
 
-// plan_next run by one warp: the independent FP64 divisions (w_d / h_d of the
-// CFL reduction, the dt / h_d coefficients) go to separate lanes.  Every
-// value keeps the expression and operation order of the serial form, so the
-// results are identical; GB300's double-precision pipe is narrow, and a
-// single thread's chain of divisions was the finalize kernel's critical path.
-__device__ __forceinline__ void plan_next_warp(const InstDesc& d, InstState& st, const double* w,
+// The next step's dt and coefficients, planned by one warp from the wave-speed
+// maxima w (python/cfdSolver/torchSession.py:379-396).  The independent
+// divisions (w_d / h_d of the CFL reduction, the dt / h_d coefficients) go to
+// separate lanes; every value keeps cfl_dt's expression and order.
+__device__ __forceinline__ void plan_next_warp(const InstDesc& d, InstState& st, const FinPre& p,
+                                               double time, int64_t steps, const double* w,
                                                int fp32, int lane) {
-  if (st.time == d.t_end) {
+  if (time == p.t_end) {
     if (lane == 0) st.status = kDone;
     return;
   }
-  if (st.steps >= d.max_steps) {
+  if (steps >= p.max_steps) {
     if (lane == 0) st.status = kErrMaxSteps;
     return;
   }
   double dt;
-  if (d.dim == 3) {
-    const double q = lane < 3 ? soft_div(w[lane], d.h[lane]) : 0.0;
+  if (d.dim == 1) {
+    const double ch = p.cfl * __shfl_sync(0xffffffffu, p.h, 0);
+    const double q = lane < 2 ? soft_div(ch, w[lane]) : 0.0;
+    const double q0 = __shfl_sync(0xffffffffu, q, 0);
+    const double dh = __shfl_sync(0xffffffffu, q, 1);
+    const double dw = soft_gt0(w[0]) ? q0 : 1e-6;
+    dt = soft_lt(dh, dw) ? dh : dw;
+  } else if (d.dim == 2 && d.bc[1] == kBcInflow) {
+    dt = cfl_dt(d, w);
+  } else {
+    const double q = lane < 3 && lane < d.dim ? soft_div(w[lane], p.h) : 0.0;
     const double q0 = __shfl_sync(0xffffffffu, q, 0);
     const double q1 = __shfl_sync(0xffffffffu, q, 1);
     const double q2 = __shfl_sync(0xffffffffu, q, 2);
-    const double total = (q0 + q1) + q2;
-    dt = soft_div(d.cfl, total);
-  } else {
-    dt = cfl_dt(d, w);
+    double total = q0 + q1;
+    if (d.dim == 3) total = total + q2;
+    dt = soft_div(p.cfl, total);
+    if (d.dim == 2 && soft_le(total, 1e-12)) dt = 1e-3;
   }
   if (fp32) dt = (double)(float)dt;
-  const double rem = d.t_end - st.time;
+  const double rem = p.t_end - time;
   if (rem < dt) dt = rem;
   if (lane < 6) {  // one division per lane: dt / h_d and half of dt over h_d
-    const int k = lane < 3 ? lane : lane - 3;
-    const double c = soft_div(lane < 3 ? soft_half(dt) : dt, d.h[k]);
-    if (lane < 3) st.coef_half[k] = c;
-    else st.coef_full[k] = c;
+    const double c = soft_div(lane < 3 ? soft_half(dt) : dt, p.h);
+    if (lane < 3) st.coef_half[lane] = c;
+    else st.coef_full[lane - 3] = c;
   } else if (lane == 6) {
     st.dt = dt;
-    st.status = (!isfinite(dt) || dt <= 0.0 || st.time + dt == st.time) ? kErrStall : kReady;
+    st.status = (!isfinite(dt) || dt <= 0.0 || time + dt == time) ? kErrStall : kReady;
   }
 }
 
@@ -1560,6 +1589,7 @@ template <typename R, int DIM, bool VARG>
 __global__ void __launch_bounds__(256) react_kernel(StepArgs A, int stage) {
   constexpr int NV = DIM + 2;
   __shared__ double red[40];
+  pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
     const Tile T = A.tiles[t];
     const InstDesc& d = A.desc[T.inst];
@@ -1681,6 +1711,7 @@ __device__ __forceinline__ R fetch_scalar(const InstDesc& d, const Geo<DIM>& g, 
 template <typename R, int DIM>
 __global__ void __launch_bounds__(256) species_kernel(StepArgs A) {
   __shared__ int red[40];
+  pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
     const Tile T = A.tiles[t];
     const InstDesc& d = A.desc[T.inst];
@@ -1750,6 +1781,7 @@ __global__ void __launch_bounds__(256) species_kernel(StepArgs A) {
 // gamma(lambda) of the current state into the per-cell gamma buffer.
 template <typename R>
 __global__ void gamma_kernel(StepArgs A) {
+  pdl_wait();
   for (int i = blockIdx.y; i < A.ninst; i += gridDim.y) {
     const InstDesc& d = A.desc[i];
     const InstState& st = A.st[i];
@@ -1779,10 +1811,13 @@ __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(StepArgs A, 
   __shared__ double sh_v[NV];
   __shared__ int fred[kFinalizeThreads / 32];
   __shared__ int sh_f, sh_last;
+  pdl_wait();
   const int i = blockIdx.y;
   if (i >= A.ninst) return;
   const InstDesc& d = A.desc[i];
   InstState& st = A.st[i];
+  FinPre pre;
+  if (threadIdx.x < 32) pre = fin_load(d, st, threadIdx.x);
   if (mode == 0 && st.status != kReady) return;  // uniform over the instance's slices
   if (mode == 4 && st.status != kReady && st.status != kRetry) return;
   const int nslices = (d.ntiles + kFinalizeSlice - 1) / kFinalizeSlice;
@@ -1892,35 +1927,36 @@ __global__ void __launch_bounds__(kFinalizeThreads) finalize_kernel(StepArgs A, 
       }
       return;
     }
-    const double dt = st.dt;
-    if (lane < nv) {
-      double out = 0.0;
-      for (int k = 0; k < d.dim; ++k) out += soft_div(dt * d.vol, d.h[k]) * sh_s[k * 5 + lane];
-      st.boundary[lane] += out;
-      if (d.reactive) st.source[lane] += d.vol * sh_i[lane];
+    const double dt = pre.dt;
+    const double per = lane < 3 ? soft_div(dt * pre.vol, pre.h) : 0.0;  // dt vol / h_k on lane k
+    double out = 0.0;
+    for (int k = 0; k < d.dim; ++k) {
+      const double f = __shfl_sync(0xffffffffu, per, k);
+      if (lane < nv) out += f * sh_s[k * 5 + lane];
     }
-    const int fb = st.fb_word;
-    __syncwarp();
+    if (lane < nv) {
+      st.boundary[lane] = pre.boundary + out;
+      if (d.reactive) st.source[lane] = pre.source + pre.vol * sh_i[lane];
+    }
+    const double tn = pre.time + dt;
+    const double time = tn < pre.t_end ? tn : pre.t_end;
     if (lane == 0) {
-      st.cur = (st.cur + A.dst_off) % d.nring;
-      const double tn = st.time + dt;
-      st.time = tn < d.t_end ? tn : d.t_end;
-      st.steps += 1;
-      st.last_fallback = fb != 0;
-      st.fallback_steps += fb != 0;
+      const int fb = pre.fb_word != 0;
+      st.cur = (pre.cur + A.dst_off) % d.nring;
+      st.time = time;
+      st.steps = pre.steps + 1;
+      st.last_fallback = fb;
+      st.fallback_steps = pre.fallback_steps + fb;
       st.fb_word = 0;
       st.retry = 0;
     }
-    __syncwarp();
-    plan_next_warp(d, st, sh_w, fp32, lane);
+    plan_next_warp(d, st, pre, time, pre.steps + 1, sh_w, fp32, lane);
     return;
   }
   if (mode == 1 || mode == 3) {
-    if (mode == 3 && lane < 5) st.initial[lane] = lane < nv ? sh_i[lane] * d.vol : 0.0;
-    const int status = st.status;
-    if (status != kReady && status != kDone) return;  // plan-only keeps a pending error
-    __syncwarp();
-    plan_next_warp(d, st, sh_w, fp32, lane);
+    if (mode == 3 && lane < 5) st.initial[lane] = lane < nv ? sh_i[lane] * pre.vol : 0.0;
+    if (pre.status != kReady && pre.status != kDone) return;  // plan-only keeps a pending error
+    plan_next_warp(d, st, pre, pre.time, pre.steps, sh_w, fp32, lane);
     return;
   }
   if (lane != 0) return;

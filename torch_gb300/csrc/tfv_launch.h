@@ -18,6 +18,24 @@ enum : int { kOpHydro = 0, kOpFallback = 1, kOpWaves = 2, kOpReact1 = 3, kOpReac
              kOpSpecies = 5, kOpGamma = 6, kOpWavesStep = 7,
              kOpStep1d = 8, kOpWavesFallback = 9, kOpWavesPlan = 10 };
 
+// Launch that may overlap the end of its predecessor on the stream: the
+// kernel waits for it (pdl_wait) before it touches shared data.
+template <typename... P, typename... Q>
+cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                       Q... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // lim selects the limiter instantiation of the step kernel (ignored otherwise).
 cudaError_t launch_step1_f64(int op, bool varg, int lim, const StepArgs& A, int grid, int block,
                              cudaStream_t s);
