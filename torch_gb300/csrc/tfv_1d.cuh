@@ -331,12 +331,14 @@ __global__ void __launch_bounds__(256) waves1d_kernel(StepArgs A, int in_step) {
 
 // Limited half-step states (left ol, right orr) of a cell with state c0
 // between neighbours cm and cp (python/cfdSolver/torchSolver.py:412-491).
+// -(dt / (2 dx)) of the Hancock half step: coef_half is (dt / 2) / dx, the same
+// quotient (both scalings by two are exact)
 template <typename R>
-__device__ __forceinline__ R recon1_coef(const InstDesc& d, const InstState& st) {
-  return -R(soft_div(st.dt, soft_twice(d.h[0])));  // -(dt / (2 dx)) of the Hancock half step
+__device__ __forceinline__ R recon1_coef(const InstState& st) {
+  return -R(st.coef_half[0]);
 }
 
-// kcoef = recon1_coef(d, st), formed once per tile by the caller
+// kcoef = recon1_coef(st), formed once per tile by the caller
 template <typename R>
 __device__ __forceinline__ void recon1_cells(const InstDesc& d, const R* c0, const R* cm,
                                              const R* cp, R g, R kcoef, R* ol, R* orr) {
@@ -388,7 +390,7 @@ __device__ __forceinline__ void recon1(const InstDesc& d, const InstState& st, c
   cell1(d, U, i, c0);
   cell1(d, U, i - 1, cm);
   cell1(d, U, i + 1, cp);
-  recon1_cells<R>(d, c0, cm, cp, gamma1(d, gam, i), recon1_coef<R>(d, st), ol, orr);
+  recon1_cells<R>(d, c0, cm, cp, gamma1(d, gam, i), recon1_coef<R>(st), ol, orr);
 }
 
 // MUSCL reconstruction and half-step predictor per cell
@@ -574,8 +576,14 @@ __device__ __forceinline__ int phys1(const InstDesc& d, int k, bool& flip) {
 // are the same expressions as in the split kernels (recon1d, update1d,
 // waves1d), so results are identical.  At a periodic domain end the wrapped
 // neighbour lies outside the staged range and is evaluated from global memory.
+// Latency-bound (five phases with a barrier each; 35% of the issue slots with
+// five 128-thread CTAs per SM at 94 registers).  Single precision is compiled
+// for 64 registers (eight CTAs per SM, so that the tiles of a served batch take
+// little more than one wave) and keeps the tile scalars' conversions and the
+// boundary sums, once per thread, off the FP64 pipe: 16 tubes of 194k cells, 64
+// steps 2.10 -> 1.58 ms (six CTAs 1.66, ten 1.60).
 template <typename R, bool VARG>
-__global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
+__global__ void __launch_bounds__(256, TFV_STEP1D_MIN_BLOCKS) step1d_kernel(StepArgs A) {
   __shared__ double red[40];
   extern __shared__ __align__(16) unsigned char step1d_smem[];
   const int W = A.tx + 6;  // staged padded cells x0-3 .. x0+tx+2
@@ -584,6 +592,7 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
   R* rc = gs + W;                              // [6][W] half-step states (l, r)
   R* fx = rc + 6 * W;                          // [3][W] flux at the face left of slot k
   R* un_s = fx + 3 * W;                        // [3][tx + 2] new state of the targets
+  __shared__ R end_flux[6];                    // domain-end fluxes: face 0, face n
   const int TS = A.tx + 2;
   pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
@@ -600,7 +609,7 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
     const int ax = min(A.tx, n - T.x0);
     const int x0 = T.x0;
     const bool per = d.bc[0] == kBcPeriodic, refl = d.bc[0] == kBcReflective;
-    const R kcoef = recon1_coef<R>(d, st);
+    const R kcoef = recon1_coef<R>(st);
     // slot k <-> padded cell x0 - 3 + k
     for (int k = threadIdx.x; k < ax + 6; k += blockDim.x) {
       const int pk = x0 - 3 + k;
@@ -670,7 +679,6 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
     __syncthreads();
     // targets: slot q <-> padded x0 + q - 1, q in [0, ax + 1]
     const R kk = -R(st.coef_full[0]);
-    double bsum[3] = {0.0, 0.0, 0.0};
     bool bad = false;
     for (int q = threadIdx.x; q < ax + 2; q += blockDim.x) {
       bool flip;
@@ -699,8 +707,8 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
         for (int c = 0; c < 3; ++c) {
           if (!TFV_IN(44, j, n) || !TFV_OUTSIDE(65, Un + c * n + j, A.ws_lo, A.ws_hi)) continue;
           Un[c * n + j] = un[c];
-          if (j == 0) bsum[c] -= (double)Fm[c];
-          if (j == n - 1) bsum[c] += (double)Fp[c];
+          if (j == 0) end_flux[c] = Fm[c];
+          if (j == n - 1) end_flux[3 + c] = Fp[c];
         }
         if (!physical_cell<R, 3>(un)) bad = true;
       }
@@ -734,16 +742,17 @@ __global__ void __launch_bounds__(256) step1d_kernel(StepArgs A) {
       }
     }
     const int fl = block_or(bad ? kFlagNonphysical : 0, reinterpret_cast<int*>(red));
-    const double mws = (double)block_max(ws, red);
-    const double mwh = (double)block_max(wh, red);
-    double sm[3] = {0.0, 0.0, 0.0};
-    if (x0 == 0 || x0 + ax == n)  // boundary faces only in the end tiles (uniform)
-      for (int c = 0; c < 3; ++c) sm[c] = block_sum(bsum[c], red);
+    const R mws = block_max(ws, red);
+    const R mwh = block_max(wh, red);
     if (threadIdx.x == 0) {
-      A.t_wmax[(size_t)t * 3 + 0] = mws;
-      A.t_wmax[(size_t)t * 3 + 1] = mwh;
+      A.t_wmax[(size_t)t * 3 + 0] = (double)mws;
+      A.t_wmax[(size_t)t * 3 + 1] = (double)mwh;
       A.t_wmax[(size_t)t * 3 + 2] = 0.0;
-      for (int c = 0; c < 3; ++c) A.t_bsum[(size_t)t * 15 + c] = sm[c];
+      // boundary faces only in the end tiles; the last face minus the first
+      for (int c = 0; c < 3; ++c) {
+        const double hi = x0 + ax == n ? (double)end_flux[3 + c] : 0.0;
+        A.t_bsum[(size_t)t * 15 + c] = x0 == 0 ? hi - (double)end_flux[c] : hi;
+      }
       A.t_flags[t] = fl;
       if (fl) atomicOr(&st.fb_word, fl);
     }

@@ -13,6 +13,7 @@
 #define TFV_LAUNCH2_NAME launch_step2_f64
 #define TFV_HLLC_NAME launch_hllc_f64
 #define TFV_WITH_1D 1
+#define TFV_STEP1D_MIN_BLOCKS 2
 #define TFV_LAUNCH1_NAME launch_step1_f64
 #define TFV_CHECK_READ_NAME check_read_f64
 #define TFV_OCC2_NAME occupancy2_f64

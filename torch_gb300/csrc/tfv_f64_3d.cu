@@ -10,6 +10,7 @@
 #define TFV_WITH_3D 1
 #define TFV_LAUNCH3_NAME launch_step3_f64
 #define TFV_WITH_1D 0
+#define TFV_STEP1D_MIN_BLOCKS 1
 #define TFV_CHECK_READ_NAME check_read_f64_3d
 #define TFV_OCC3_NAME occupancy3_f64
 #include "tfv_inst.inc"
