@@ -174,10 +174,21 @@ struct Driver {
   const void* prim_state = nullptr;
   int prim_slot = -1;
 
-  cudaError_t launch(int op, int arg, int grid) {
+  cudaError_t launch(int op, int arg, int grid, int block = 256) {
     return sizeof(R) == 8
-               ? metric_launch_f64(op, m->dim, reinterpret_cast<const MArgs<double>&>(A), arg, grid, s)
-               : metric_launch_f32(op, m->dim, reinterpret_cast<const MArgs<float>&>(A), arg, grid, s);
+               ? metric_launch_f64(op, m->dim, reinterpret_cast<const MArgs<double>&>(A), arg, grid,
+                                   block, s)
+               : metric_launch_f32(op, m->dim, reinterpret_cast<const MArgs<float>&>(A), arg, grid,
+                                   block, s);
+  }
+  // a face or march launch over `work` threads: double precision in 64-thread
+  // CTAs, whose registers leave two 256-thread CTAs to an SM (a grid of a few
+  // hundred large CTAs would load some SMs twice as much as others)
+  cudaError_t launch_work(int op, int arg, int64_t work) {
+    if (sizeof(R) != 8) return launch(op, arg, grid_for(m, work));
+    const int64_t blocks = (work + 63) / 64;
+    return launch(op, arg, (int)std::max<int64_t>(1, std::min<int64_t>(blocks, (int64_t)m->sms * 32)),
+                  64);
   }
   void set_input(const View& v) {
     A.U = (const R*)v.u;
@@ -231,15 +242,20 @@ struct Driver {
       } else if (d > 0 || (m->dim >= 2 && m->esz == 8)) {
         const int64_t lines = m->nc / m->cfg.n[d];
         const int64_t runs = m->cfg.n[d] + (last_fused ? 0 : 1);
-        const int64_t target = (int64_t)m->sms * 8 * 256;
+        // double precision: about 16 warps per SM are resident, and a run of
+        // c faces forms c + 1 slopes, so short runs only where the grid leaves
+        // SMs idle (annulus 256 x 192, 4 steps: 1.44 ms with 48 CTAs of
+        // four-face runs, 1.06 with two, 1.01 with one face a thread)
+        const bool d64 = m->esz == 8;
+        const int64_t target = (int64_t)m->sms * (d64 ? 512 : 8 * 256);
         A.chunk = (int)std::max<int64_t>(
-            4, std::min<int64_t>(kMChunk, (runs * lines + target - 1) / target));
+            d64 ? 1 : 4, std::min<int64_t>(kMChunk, (runs * lines + target - 1) / target));
         work = lines * ((runs + A.chunk - 1) / A.chunk);
       }
       if (last_fused)
-        TFV_MCUDA(launch(kMOpMarchUpdate, stage, grid_for(m, work)));
+        TFV_MCUDA(launch_work(kMOpMarchUpdate, stage, work));
       else
-        TFV_MCUDA(launch(kMOpFace, d, grid_for(m, work)));
+        TFV_MCUDA(launch_work(kMOpFace, d, work));
     }
     int64_t plane = 0;
     for (int d = 0; d < m->dim; ++d) plane = std::max<int64_t>(plane, m->nc / m->cfg.n[d]);

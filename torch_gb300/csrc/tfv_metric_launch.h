@@ -20,9 +20,9 @@ enum : int {
 };
 
 cudaError_t metric_launch_f64(int op, int dim, const MArgs<double>& A, int arg, int grid,
-                              cudaStream_t s);
+                              int block, cudaStream_t s);
 cudaError_t metric_launch_f32(int op, int dim, const MArgs<float>& A, int arg, int grid,
-                              cudaStream_t s);
+                              int block, cudaStream_t s);
 // Rusanov fluxes of n faces (rows [nv][n], primitive face states)
 cudaError_t rusanov_launch_f64(int nv, int64_t n, int dir, const void* l, const void* r,
                                const void* gl, const void* gr, void* out, int grid,
