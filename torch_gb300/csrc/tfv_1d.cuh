@@ -521,6 +521,110 @@ __global__ void __launch_bounds__(256) update1d_kernel(StepArgs A, int first_ord
 }
 
 
+// Reaction half step over every tile.  stage 1: start (ring cur) -> heated
+// (cur+1) and gamma(lambda) for the hydro step.  stage 2: hydro (cur+2) -> new
+// (cur+1, where the heated state was), source partial sums (old - start + new -
+// hydro) (python/cfdSolver/torchSession.py:401-411, 510-517).
+template <typename R, bool VARG>
+__global__ void __launch_bounds__(256) react1d_kernel(StepArgs A, int stage) {
+  __shared__ double red[40];
+  pdl_wait();
+  for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
+    const Tile T = A.tiles[t];
+    const InstDesc& d = A.desc[T.inst];
+    InstState& st = A.st[T.inst];
+    const int status = st.status;
+    if (!(status == kReady || (stage == 1 && status == kRetry))) continue;  // uniform
+    const int n = d.n[0];
+    const int cur = st.cur;
+    const int i0 = cur % d.nring, i1 = (cur + 1) % d.nring, i2 = (cur + 2) % d.nring;
+    const int is = stage == 1 ? i0 : i2;
+    const R* Usrc = (const R*)d.U[is];
+    R* Udst = (R*)d.U[i1];
+    const R* Ustart = (const R*)d.U[i0];
+    const bool znd = d.model == 1;
+    const Chem<R> chem(d);
+    const int i = T.x0 + (int)threadIdx.x;
+    const bool owner = (int)threadIdx.x < min(A.tx, n - T.x0);
+    R wmax = R(0);
+    double src[3] = {0.0, 0.0, 0.0};
+    int fl = 0;
+    if (owner) {
+      R u[3], hyd[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) u[c] = hyd[c] = Usrc[c * n + i];
+      R lam = ((const R*)d.lam[is])[i];
+      R beta = znd ? ((const R*)d.beta[is])[i] : R(1);
+      if (!react_cell<R, 1>(chem, u, lam, beta, znd, 0.5 * st.dt)) fl |= kFlagChemistry;
+      if (stage == 2) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const R old = Udst[c * n + i];  // heated state of this step
+          const R start = Ustart[c * n + i];
+          src[c] = (double)(((old - start) + u[c]) - hyd[c]);
+        }
+        if (!physical_cell<R, 3>(u)) fl |= kFlagNonphysical;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) Udst[c * n + i] = u[c];
+      ((R*)d.lam[i1])[i] = lam;
+      if (znd) ((R*)d.beta[i1])[i] = beta;
+      const R gc = (chem.closure == 0) ? gamma_of_lambda(lam) : chem.gamma;
+      if (VARG && stage == 1) ((R*)d.gam)[i] = gc;
+      wave_speeds<R, 1>(u, gc, &wmax);
+      wmax = run_max(R(0), wmax);
+    }
+    fl = block_or(fl, reinterpret_cast<int*>(red));
+    const R wm = block_max(wmax, red);
+    double sm[3] = {0.0, 0.0, 0.0};
+    if (stage == 2)  // uniform
+      for (int c = 0; c < 3; ++c) sm[c] = block_sum(src[c], red);
+    if (threadIdx.x == 0) {
+      A.t_wmax[(size_t)t * 3] = (double)wm;
+      if (stage == 2) {
+        for (int c = 0; c < 3; ++c) A.t_sum[(size_t)t * 5 + c] = sm[c];
+        A.t_flags[t] |= fl;
+      } else {
+        A.t_flags[t] = fl;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// Species transport with the interface mass fluxes, first-order upwind
+// (python/cfdSolver/torchSolver.py:1125-1132): lambda (and beta) of the heated
+// state (ring cur+1) -> ring cur+2.
+template <typename R>
+__global__ void __launch_bounds__(256) species1d_kernel(StepArgs A) {
+  pdl_wait();
+  for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
+    const Tile T = A.tiles[t];
+    const InstDesc& d = A.desc[T.inst];
+    const InstState& st = A.st[T.inst];
+    if (st.status != kReady) continue;  // uniform
+    Geo<1> g;
+    g.init(d);
+    const int i1 = (st.cur + 1) % d.nring, i2 = (st.cur + 2) % d.nring;
+    const int i = T.x0 + (int)threadIdx.x;
+    if ((int)threadIdx.x >= min(A.tx, g.na - T.x0)) continue;
+    const R* F = (const R*)d.flux_out[0];
+    const R Flo = F[i], Fhi = F[i + 1], k = R(st.coef_full[0]);
+    const R rho = ((const R*)d.U[i1])[i], rhon = floored(((const R*)d.U[i2])[i]);
+    const int nq = d.model == 1 ? 2 : 1;
+    for (int s = 0; s < nq; ++s) {
+      const R* q = (const R*)(s == 0 ? d.lam[i1] : d.beta[i1]);
+      const R qc = q[i];
+      const R ql = fetch_scalar<R, 1>(d, g, q, i - 1, 0, 0);
+      const R qr = fetch_scalar<R, 1>(d, g, q, i + 1, 0, 0);
+      const R Glo = Flo * (ge0(Flo) ? ql : qc);
+      const R Ghi = Fhi * (ge0(Fhi) ? qc : qr);
+      const R f = qd(rho * qc - k * (Ghi - Glo), rhon);
+      ((R*)(s == 0 ? d.lam[i2] : d.beta[i2]))[i] = np_min(np_max(f, R(0)), R(1));
+    }
+  }
+}
+
 // Face flux at face f (0 <= f <= n) of the current state, evaluated from
 // scratch: the two reconstructed interface states (bc_creator rules at the
 // domain faces, torchSolver.py:494-508), the interface wave speeds

@@ -599,8 +599,10 @@ cudaError_t finalize(tfv_batch* b, int mode, int dst_off) {
 // state (ring cur -> cur+1) and the CFL check, which may halve dt and leave
 // the instance in RETRY (the next enqueued step retries from the start
 // state); hydro on the heated state (cur+1 -> cur+2) with its mass fluxes;
-// species transport; second half reaction (cur+2 -> cur+1) with the source
-// sums; commit (cur <- cur+1).
+// species transport and the second half reaction with the source sums; commit.
+// 2D / 3D: transport and reaction are one kernel that reacts the hydro state in
+// place (cur <- cur+2); the 1D chain writes the new state over the heated one
+// (cur+2 -> cur+1, cur <- cur+1).
 cudaError_t enqueue_step(tfv_batch* b) {
   if (b->dim == 1) {  // the 1D chain: wave speeds of the new state plan the next dt
     cudaError_t e = cudaSuccess;
@@ -630,9 +632,8 @@ cudaError_t enqueue_step(tfv_batch* b) {
     if (e == cudaSuccess) e = finalize(b, 4, 1);
     if (e == cudaSuccess) e = launch(b, kOpHydro, 1, 2);
     if (e == cudaSuccess) e = launch(b, kOpFallback, 1, 2);
-    if (e == cudaSuccess) e = launch(b, kOpSpecies, 1, 2);
-    if (e == cudaSuccess) e = launch(b, kOpReact2, 2, 1);
-    if (e == cudaSuccess) e = finalize(b, 0, 1);
+    if (e == cudaSuccess) e = launch(b, kOpReact2, 2, 2);
+    if (e == cudaSuccess) e = finalize(b, 0, 2);
     return e;
   }
   cudaError_t e = launch(b, kOpHydro, 0, 1);

@@ -1579,15 +1579,21 @@ __device__ __forceinline__ bool react_cell(const Chem<R>& d, R* u, R& lam, R& be
   return ok;
 }
 
-// Reaction half step over every tile.  stage 1: start (ring cur) -> heated
+// First reaction half step of 2D / 3D tiles: start (ring cur) -> heated
 // (cur+1) and gamma(lambda) for the hydro step; wave maxima for the reactive
-// dt check.  stage 2: hydro (cur+2) -> new (cur+1, where the heated state
-// was), source partial sums (old - start + new - hydro) and the wave maxima of
-// the new state for the next dt (python/cfdSolver/torchSession.py:401-411,
-// 510-517).
+// dt check (python/cfdSolver/torchSession.py:401-411).  Bound by HBM: the state
+// and the fractions read and written once, 48 B per cell in single precision.
+// A thread walks a column of its tile; the loads of kHeatPlanes planes are
+// issued before the first is used (one plane at a time left the loop waiting
+// for memory: 192^3, 162 us a launch against 50 us of traffic; now 62).
+template <typename R>
+struct HeatPlanes {
+  static constexpr int value = sizeof(R) == 4 ? 4 : 2;
+};
 template <typename R, int DIM, bool VARG>
-__global__ void __launch_bounds__(256) react_kernel(StepArgs A, int stage) {
+__global__ void __launch_bounds__(256) heat_kernel(StepArgs A) {
   constexpr int NV = DIM + 2;
+  constexpr int G = HeatPlanes<R>::value;
   __shared__ double red[40];
   pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
@@ -1595,19 +1601,17 @@ __global__ void __launch_bounds__(256) react_kernel(StepArgs A, int stage) {
     const InstDesc& d = A.desc[T.inst];
     InstState& st = A.st[T.inst];
     const int status = st.status;
-    if (!(status == kReady || (stage == 1 && status == kRetry))) continue;  // uniform
+    if (status != kReady && status != kRetry) continue;  // uniform
     Geo<DIM> g;
     g.init(d);
-    const int cur = st.cur;
-    const int i0 = cur % d.nring, i1 = (cur + 1) % d.nring, i2 = (cur + 2) % d.nring;
-    const R* Usrc = (const R*)d.U[stage == 1 ? i0 : i2];
-    R* Udst = (R*)d.U[i1];
-    const R* Ustart = (const R*)d.U[i0];
-    const R* Lsrc = (const R*)d.lam[stage == 1 ? i0 : i2];
-    R* Ldst = (R*)d.lam[i1];
+    const int i0 = st.cur % d.nring, i1 = (st.cur + 1) % d.nring;
+    const R* U = (const R*)d.U[i0];
+    R* Un = (R*)d.U[i1];
+    const R* L = (const R*)d.lam[i0];
+    R* Ln = (R*)d.lam[i1];
     const bool znd = d.model == 1;
-    const R* Bsrc = znd ? (const R*)d.beta[stage == 1 ? i0 : i2] : nullptr;
-    R* Bdst = znd ? (R*)d.beta[i1] : nullptr;
+    const R* B = znd ? (const R*)d.beta[i0] : nullptr;
+    R* Bn = znd ? (R*)d.beta[i1] : nullptr;
     R* gam = VARG ? (R*)d.gam : nullptr;
     const double half = 0.5 * st.dt;
     const Chem<R> chem(d);
@@ -1619,84 +1623,49 @@ __global__ void __launch_bounds__(256) react_kernel(StepArgs A, int stage) {
     R wmax[DIM];
 #pragma unroll
     for (int k = 0; k < DIM; ++k) wmax[k] = R(0);
-    double src[NV];
-#pragma unroll
-    for (int c = 0; c < NV; ++c) src[c] = 0.0;
-    // single precision: this thread's column of source terms summed with
-    // compensation (Kahan), converted once; the tile and global sums are FP64
-    R ksum[NV], kcomp[NV];
-#pragma unroll
-    for (int c = 0; c < NV; ++c) ksum[c] = kcomp[c] = R(0);
     int fl = 0;
     if (owner) {
-      for (int p = T.p0; p < T.p1; ++p) {
-        const int64_t off = (int64_t)p * g.ps + (int64_t)b * g.na + a;
-        R u[NV], hyd[NV];
+      for (int p = T.p0; p < T.p1; p += G) {
+        R u[G][NV], lam[G], beta[G];
 #pragma unroll
-        for (int c = 0; c < NV; ++c) {
-          u[c] = Usrc[c * g.cs + off];
-          hyd[c] = u[c];
-        }
-        R lam = Lsrc[off];
-        R beta = znd ? Bsrc[off] : R(1);
-        if (!react_cell<R, DIM>(chem, u, lam, beta, znd, half)) fl |= kFlagChemistry;
-        if (stage == 2) {
+        for (int q = 0; q < G; ++q) {
+          const int64_t off = (int64_t)min(p + q, T.p1 - 1) * g.ps + (int64_t)b * g.na + a;
 #pragma unroll
-          for (int c = 0; c < NV; ++c) {
-            if constexpr (Exact<R>::value) {
-              const double old = Udst[c * g.cs + off];  // heated state of this step
-              const double start = Ustart[c * g.cs + off];
-              src[c] += ((old - start) + u[c]) - hyd[c];
-            } else {
-              const R old = Udst[c * g.cs + off];
-              const R start = Ustart[c * g.cs + off];
-              const R y = (((old - start) + u[c]) - hyd[c]) - kcomp[c];
-              const R t = ksum[c] + y;
-              kcomp[c] = (t - ksum[c]) - y;
-              ksum[c] = t;
-            }
-          }
-          if (!physical_cell<R, NV>(u)) fl |= kFlagNonphysical;
+          for (int c = 0; c < NV; ++c) u[q][c] = U[c * g.cs + off];
+          lam[q] = L[off];
+          beta[q] = znd ? B[off] : R(1);
         }
 #pragma unroll
-        for (int c = 0; c < NV; ++c) Udst[c * g.cs + off] = u[c];
-        Ldst[off] = lam;
-        if (znd) Bdst[off] = beta;
-        const R gc = (chem.closure == 0) ? gamma_of_lambda(lam) : chem.gamma;
-        if (VARG && stage == 1) gam[off] = gc;
-        R w[DIM];
-        wave_speeds<R, DIM>(u, gc, w);
+        for (int q = 0; q < G; ++q) {
+          if (p + q >= T.p1) break;
+          const int64_t off = (int64_t)(p + q) * g.ps + (int64_t)b * g.na + a;
+          if (!react_cell<R, DIM>(chem, u[q], lam[q], beta[q], znd, half)) fl |= kFlagChemistry;
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
+          for (int c = 0; c < NV; ++c) Un[c * g.cs + off] = u[q][c];
+          Ln[off] = lam[q];
+          if (znd) Bn[off] = beta[q];
+          const R gc = (chem.closure == 0) ? gamma_of_lambda(lam[q]) : chem.gamma;
+          if (VARG) gam[off] = gc;
+          R w[DIM];
+          wave_speeds<R, DIM>(u[q], gc, w);
+#pragma unroll
+          for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
+        }
       }
     }
     fl = block_or(fl, reinterpret_cast<int*>(red));
-    double wm[DIM], sm[NV];
+    R wm[DIM];
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) wm[k] = (double)block_max(owner ? wmax[k] : R(0), red);
-#pragma unroll
-    for (int c = 0; c < NV; ++c) {
-      if constexpr (!Exact<R>::value) src[c] = (double)ksum[c] - (double)kcomp[c];
-      sm[c] = stage == 2 ? block_sum(src[c], red) : 0.0;
-    }
+    for (int k = 0; k < DIM; ++k) wm[k] = block_max(owner ? wmax[k] : R(0), red);
     if (threadIdx.x == 0) {
-      for (int k = 0; k < DIM; ++k) A.t_wmax[(size_t)t * 3 + k] = wm[k];
-      if (stage == 2) {
-        for (int c = 0; c < NV; ++c) A.t_sum[(size_t)t * 5 + c] = sm[c];
-        A.t_flags[t] |= fl;
-      } else {
-        A.t_flags[t] = fl;
-      }
+      for (int k = 0; k < DIM; ++k) A.t_wmax[(size_t)t * 3 + k] = (double)wm[k];
+      A.t_flags[t] = fl;
     }
     __syncthreads();
   }
 }
 
-// Species transport with the hydro mass fluxes: first-order upwind in every
-// direction (python/cfdSolver/torchSolver3D.py:246-256,
-// torchSolver2D.py:659-667).  q = lambda (and beta) of the heated state
-// (ring cur+1) -> ring cur+2.  Scalar ghost cells: no sign change; the 2D
-// inlet rows hold fresh mixture (1).
+// Scalar ghost cells: no sign change; the 2D inlet rows hold fresh mixture (1).
 template <typename R, int DIM>
 __device__ __forceinline__ R fetch_scalar(const InstDesc& d, const Geo<DIM>& g, const R* q, int a,
                                           int b, int p) {
@@ -1708,9 +1677,25 @@ __device__ __forceinline__ R fetch_scalar(const InstDesc& d, const Geo<DIM>& g, 
   return q[(int64_t)sp * g.ps + (int64_t)sb * g.na + sa];
 }
 
-template <typename R, int DIM>
-__global__ void __launch_bounds__(256) species_kernel(StepArgs A) {
-  __shared__ int red[40];
+// Species transport with the hydro mass fluxes and the closing reaction half
+// step of 2D / 3D tiles, in one pass: first-order upwind transport of lambda
+// (and beta) in every direction (python/cfdSolver/torchSolver3D.py:246-256,
+// torchSolver2D.py:659-667) from the heated fractions (ring cur+1), then the
+// reaction on the hydro state in place (cur+2, which becomes the new state:
+// only its energy changes), the source sums (old - start + new - hydro,
+// python/cfdSolver/torchSession.py:510-517) and the wave maxima of the new
+// state.  The reaction moves energy only, so the sums of the other components
+// are zero and their heated and start states are not read.  56 B per cell in
+// single precision against 116 of a transport and a reaction pass (192^3: 142 +
+// 162 us for the two before).  A thread walks a column, the loads of a plane
+// issued together; three CTAs per SM in single precision (192^3, ten attempts:
+// 4.14 ms; two CTAs 4.40).
+template <typename R, int DIM, bool VARG>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) burn_kernel(StepArgs A) {
+  constexpr int NV = DIM + 2;
+  constexpr int E = NV - 1;
+  constexpr int MD = DIM - 1;
+  __shared__ double red[40];
   pdl_wait();
   for (int t = A.t_begin + blockIdx.x; t < A.t_end; t += gridDim.x) {
     const Tile T = A.tiles[t];
@@ -1720,11 +1705,17 @@ __global__ void __launch_bounds__(256) species_kernel(StepArgs A) {
     Geo<DIM> g;
     g.init(d);
     const int cur = st.cur;
-    const int i1 = (cur + 1) % d.nring, i2 = (cur + 2) % d.nring;
-    const R* Uold = (const R*)d.U[i1];
-    const R* Unew = (const R*)d.U[i2];
-    const int nq = d.model == 1 ? 2 : 1;
+    const int i0 = cur % d.nring, i1 = (cur + 1) % d.nring, i2 = (cur + 2) % d.nring;
+    R* U = (R*)d.U[i2];
+    const R* rho1 = (const R*)d.U[i1];
+    const R* e1 = rho1 + E * g.cs;
+    const R* e0 = (const R*)d.U[i0] + E * g.cs;
+    const bool znd = d.model == 1;
     const R* mf[3] = {(const R*)d.flux_out[0], (const R*)d.flux_out[1], (const R*)d.flux_out[2]};
+    const R* q1[2] = {(const R*)d.lam[i1], znd ? (const R*)d.beta[i1] : nullptr};
+    R* qn[2] = {(R*)d.lam[i2], znd ? (R*)d.beta[i2] : nullptr};
+    const double half = 0.5 * st.dt;
+    const Chem<R> chem(d);
     R cu[DIM];
 #pragma unroll
     for (int k = 0; k < DIM; ++k) cu[k] = R(st.coef_full[k]);
@@ -1733,47 +1724,138 @@ __global__ void __launch_bounds__(256) species_kernel(StepArgs A) {
     const bool owner = (int)threadIdx.x < ax * by;
     const int a = T.x0 + (owner ? (int)threadIdx.x % ax : 0);
     const int b = DIM == 3 ? T.y0 + (owner ? (int)threadIdx.x / ax : 0) : 0;
+    R wmax[DIM];
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) wmax[k] = R(0);
+    // energy source of this thread's column: double, or single with Kahan's
+    // compensation, converted once (the tile and global sums are FP64)
+    double src = 0.0;
+    R ksum = R(0), kcomp = R(0);
     int fl = 0;
     if (owner) {
-      for (int s = 0; s < nq; ++s) {
-        const R* q = (const R*)(s == 0 ? d.lam[i1] : d.beta[i1]);
-        R* qn = (R*)(s == 0 ? d.lam[i2] : d.beta[i2]);
-        for (int p = T.p0; p < T.p1; ++p) {
-          const int64_t off = (int64_t)p * g.ps + (int64_t)b * g.na + a;
-          const R qc = q[off];
-          R rhoq = Uold[off] * qc;
+      // what one plane of the column reads: the hydro state, the heated and
+      // start energies, the heated density, the in-plane mass fluxes (low,
+      // high) and in-plane upwind neighbours, the high marching flux and the
+      // plane above
+      struct Plane {
+        R u[NV], e1, e0, rho, f[2 * MD], fz, q[2][2 * MD], qz[2];
+      };
+      // in-plane neighbours by the boundary mapping, the same for every plane;
+      // running offsets of the column's cell and faces
+      bool ghost;
+      const int64_t row = (int64_t)b * g.na;
+      const int64_t oq[4] = {row + map_axis(a - 1, g.na, g.bca, ghost),
+                             row + map_axis(a + 1, g.na, g.bca, ghost),
+                             DIM == 3 ? (int64_t)map_axis(b - 1, g.nb, g.bcb, ghost) * g.na + a : 0,
+                             DIM == 3 ? (int64_t)map_axis(b + 1, g.nb, g.bcb, ghost) * g.na + a : 0};
+      const int64_t dfx = (int64_t)g.nb * (g.na + 1), dfy = (int64_t)(g.nb + 1) * g.na;
+      int64_t plane = (int64_t)T.p0 * g.ps;
+      int64_t fx = T.p0 * dfx + (int64_t)b * (g.na + 1) + a;
+      int64_t fy = T.p0 * dfy + row + a;
+      auto load = [&](int p, Plane& P) {
+        const int64_t off = plane + row + a;
+#pragma unroll
+        for (int c = 0; c < NV; ++c) P.u[c] = U[c * g.cs + off];
+        P.e1 = e1[off];
+        P.e0 = e0[off];
+        P.rho = rho1[off];
+        P.f[0] = mf[0][fx];
+        P.f[1] = mf[0][fx + 1];
+        if (DIM == 3) {
+          P.f[2] = mf[1][fy];
+          P.f[3] = mf[1][fy + g.na];
+        }
+        P.fz = mf[MD][off + g.ps];
+        const int64_t above = (int64_t)map_axis(p + 1, g.np, g.bcp, ghost) * g.ps + row + a;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (s == 1 && !znd) break;
+#pragma unroll
+          for (int k = 0; k < 2 * MD; ++k) P.q[s][k] = q1[s][plane + oq[k]];
+          P.qz[s] = q1[s][above];
+        }
+      };
+      R qlo[2], qc[2];
+      const int64_t off0 = plane + row + a;
+#pragma unroll
+      for (int s = 0; s < 2; ++s) {
+        qlo[s] = qc[s] = R(1);
+        if (s == 1 && !znd) break;
+        qlo[s] = fetch_scalar<R, DIM>(d, g, q1[s], a, b, T.p0 - 1);
+        qc[s] = q1[s][off0];
+      }
+      R flo = mf[MD][off0];
+      Plane P;
+      for (int p = T.p0; p < T.p1; ++p) {
+        load(p, P);
+        const int64_t off = plane + row + a;
+        plane += g.ps;
+        fx += dfx;
+        fy += dfy;
+        R frac[2] = {R(1), R(1)};
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          if (s == 1 && !znd) break;
+          R rhoq = P.rho * qc[s];
 #pragma unroll
           for (int dd = 0; dd < DIM; ++dd) {
-            const int ia = dd == 0 ? 1 : 0;
-            const int ib = (DIM == 3 && dd == 1) ? 1 : 0;
-            const int ip = (DIM > 1 && dd == DIM - 1) ? 1 : 0;  // 1D has no marching axis
-            // face arrays of this direction have one more entry along dd
-            const int fa_n = dd == 0 ? g.na + 1 : g.na;
-            const int fb_n = (DIM == 3 && dd == 1) ? g.nb + 1 : g.nb;
-            const int64_t lo = ((int64_t)p * fb_n + b) * fa_n + a;
-            const int64_t hi = ((int64_t)(p + ip) * fb_n + b + ib) * fa_n + a + ia;
-            const R Flo = mf[dd][lo], Fhi = mf[dd][hi];
-            const R qlo_l = fetch_scalar<R, DIM>(d, g, q, a - ia, b - ib, p - ip);
-            const R qhi_r = fetch_scalar<R, DIM>(d, g, q, a + ia, b + ib, p + ip);
-            const R Glo = Flo * (ge0(Flo) ? qlo_l : qc);
-            const R Ghi = Fhi * (ge0(Fhi) ? qc : qhi_r);
+            const R Flo = dd == MD ? flo : P.f[dd < MD ? 2 * dd : 0];
+            const R Fhi = dd == MD ? P.fz : P.f[dd < MD ? 2 * dd + 1 : 0];
+            const R ql = dd == MD ? qlo[s] : P.q[s][dd < MD ? 2 * dd : 0];
+            const R qr = dd == MD ? P.qz[s] : P.q[s][dd < MD ? 2 * dd + 1 : 0];
+            const R Glo = Flo * (ge0(Flo) ? ql : qc[s]);
+            const R Ghi = Fhi * (ge0(Fhi) ? qc[s] : qr);
             rhoq = rhoq - cu[dd] * (Ghi - Glo);
           }
-          R frac;
+          R f;
           if (DIM == 3) {
             // the reference's interval check; FP32 roundoff needs a wider margin
             const R tol = Exact<R>::value ? R(1e-10) : R(1e-5);
-            frac = qd(rhoq, Unew[off]);
-            if (lt_(frac, -tol) || gt_pos(frac, R(1) + tol)) fl |= kFlagSpecies;
+            f = qd(rhoq, P.u[0]);
+            if (lt_(f, -tol) || gt_pos(f, R(1) + tol)) fl |= kFlagSpecies;
           } else {
-            frac = qd(rhoq, floored(Unew[off]));
+            f = qd(rhoq, floored(P.u[0]));
           }
-          qn[off] = np_min(np_max(frac, R(0)), R(1));
+          frac[s] = np_min(np_max(f, R(0)), R(1));
+        }
+        const R hyd = P.u[E];
+        if (!react_cell<R, DIM>(chem, P.u, frac[0], frac[1], znd, half)) fl |= kFlagChemistry;
+        if constexpr (Exact<R>::value) {
+          src += ((P.e1 - P.e0) + P.u[E]) - hyd;
+        } else {
+          const R y = (((P.e1 - P.e0) + P.u[E]) - hyd) - kcomp;
+          const R v = ksum + y;
+          kcomp = (v - ksum) - y;
+          ksum = v;
+        }
+        if (!physical_cell<R, NV>(P.u)) fl |= kFlagNonphysical;
+        U[E * g.cs + off] = P.u[E];
+        qn[0][off] = frac[0];
+        if (znd) qn[1][off] = frac[1];
+        const R gc = (chem.closure == 0) ? gamma_of_lambda(frac[0]) : chem.gamma;
+        R w[DIM];
+        wave_speeds<R, DIM>(P.u, gc, w);
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) wmax[k] = run_max(wmax[k], w[k]);
+        flo = P.fz;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          qlo[s] = qc[s];
+          if (s == 0 || znd) qc[s] = P.qz[s];
         }
       }
     }
-    fl = block_or(fl, red);
-    if (threadIdx.x == 0 && fl) atomicOr(&A.t_flags[t], fl);
+    fl = block_or(fl, reinterpret_cast<int*>(red));
+    R wm[DIM];
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) wm[k] = block_max(owner ? wmax[k] : R(0), red);
+    if constexpr (!Exact<R>::value) src = (double)ksum - (double)kcomp;
+    const double sm = block_sum(src, red);
+    if (threadIdx.x == 0) {
+      for (int k = 0; k < DIM; ++k) A.t_wmax[(size_t)t * 3 + k] = (double)wm[k];
+      for (int c = 0; c < NV; ++c) A.t_sum[(size_t)t * 5 + c] = c == E ? sm : 0.0;
+      A.t_flags[t] |= fl;
+    }
     __syncthreads();
   }
 }

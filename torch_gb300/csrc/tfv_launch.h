@@ -12,7 +12,8 @@ namespace tfv {
 // kOpWavesStep: the 1D chain's wave-speed pass inside a step (keeps the step's
 // source sums and ORs its flags into those of the earlier kernels);
 // kOpStep1d: the fused inert 1D step; kOpWavesFallback: the wave-speed pass
-// for the instances whose step was redone at first order; kOpWavesPlan: wave
+// for the instances whose step was redone at first order; kOpSpecies: the 1D
+// transport (2D / 3D: part of kOpReact2); kOpWavesPlan: wave
 // maxima and flags of the current state without its integrals (re-planning)
 enum : int { kOpHydro = 0, kOpFallback = 1, kOpWaves = 2, kOpReact1 = 3, kOpReact2 = 4,
              kOpSpecies = 5, kOpGamma = 6, kOpWavesStep = 7,
