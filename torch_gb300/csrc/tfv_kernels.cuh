@@ -279,6 +279,9 @@ __device__ __forceinline__ void copy_async(float* dst, const float* src) {
 __device__ __forceinline__ void copy_async(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
+__device__ __forceinline__ void copy_async2(float* dst, const float* src) {  // 8-byte aligned
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // --------------------------------------------------------------------------
@@ -388,41 +391,65 @@ struct HydroTile {
   // Start copying the in-domain cells of in-range plane p (2-cell in-plane
   // halo) into `dst` asynchronously: the grids whose row pitch rules out a
   // tensor copy (x extent not a multiple of 16 bytes).  One cp.async per
-  // element, one warp per staged row; fix_ghosts fills the cells outside the
-  // domain.  Loads through registers had to wait for their data before the
-  // plane's faces could start, and edge tiles took the boundary mapping for
-  // every cell (FP32 batch of six 3D grids of 68 to 154 cells a side, four of
-  // them odd: 11.53 -> 8.78 ms per 8 steps).
-  static __device__ __forceinline__ void copy_plane(const Geo<DIM>& g, const R* U, const R* gam,
-                                                    R* dst, const HydroSmem<R, DIM, VARG>& S,
-                                                    int x0, int y0, int ax, int by, int p) {
-    const int w = min(ax + 4, g.na - x0 + 2);   // staged columns la0 .. w - 1 lie in the domain
-    const int la0 = x0 == 0 ? 2 : 0;
-    const int h = DIM == 3 ? by + 4 : 1;
-    const int lb0 = DIM == 3 && y0 == 0 ? 2 : 0;
-    const int rows = (DIM == 3 ? min(h, g.nb - y0 + 2) : 1) - lb0;  // rows in the domain
+  // element, or per pair where a single-precision row starts on 8 bytes;
+  // fix_ghosts fills the cells outside the domain.  Loads through registers had
+  // to wait for their data before the plane's faces could start, and edge tiles
+  // took the boundary mapping for every cell (FP32 batch of six 3D grids of 68
+  // to 154 cells a side, three of them odd: 11.53 -> 8.78 ms per 8 steps).  The
+  // staged rows are walked as one run of elements, thread after thread, row and
+  // column advanced by constant steps: a warp per row left 12 of 32 lanes idle
+  // and spent a loop on each row (8.31 -> 7.05 ms).
+  template <int V>
+  static __device__ __forceinline__ void copy_rows(const Geo<DIM>& g, const R* U, const R* gam,
+                                                   R* dst, const HydroSmem<R, DIM, VARG>& S,
+                                                   int64_t base, int la0, int lb0, int cols,
+                                                   int rows) {
     const int plane = S.ph * S.pw;
-    const int nwarps = blockDim.x >> 5;
-    const int la = la0 + (threadIdx.x & 31);
-    const int64_t base = (int64_t)p * g.ps + (DIM == 3 ? (int64_t)(y0 - 2) * g.na : 0) + (x0 - 2);
-    int c = 0, r = threadIdx.x >> 5;
+    const int w = cols / V;
+    const int drow = (int)blockDim.x / w, dcol = (int)blockDim.x - drow * w;
+    int r = (int)threadIdx.x / w;
+    int k = (int)threadIdx.x - r * w;
+    int c = 0;
     while (true) {
       while (r >= rows) {
         r -= rows;
         ++c;
       }
       if (c >= NL) break;
-      const int lb = lb0 + r;
-      const R* src = (VARG && c == NV ? gam : U + c * g.cs) + base + (int64_t)lb * g.na;
-      const int at = (VARG && c == NV ? S.goff : c * plane) + lb * S.pw + (S.xo - 2);
-      for (int k = la; k < w; k += 32) {
-        if (!TFV_IN(3, base + (int64_t)lb * g.na + k, g.cs) ||
-            !TFV_IN(4, at + k, (int64_t)S.slot_elems))
-          continue;
-        copy_async(dst + at + k, src + k);
+      const int lb = lb0 + r, la = la0 + k * V;
+      const R* src = (VARG && c == NV ? gam : U + c * g.cs) + base + (int64_t)lb * g.na + la;
+      const int at = (VARG && c == NV ? S.goff : c * plane) + lb * S.pw + (S.xo - 2) + la;
+      if (TFV_IN(3, base + (int64_t)lb * g.na + la + V - 1, g.cs) &&
+          TFV_IN(4, at + V - 1, (int64_t)S.slot_elems)) {
+        if constexpr (V == 2) copy_async2(dst + at, src);
+        else copy_async(dst + at, src);
       }
-      r += nwarps;
+      r += drow;
+      k += dcol;
+      if (k >= w) {
+        k -= w;
+        ++r;
+      }
     }
+  }
+  static __device__ __forceinline__ void copy_plane(const Geo<DIM>& g, const R* U, const R* gam,
+                                                    R* dst, const HydroSmem<R, DIM, VARG>& S,
+                                                    int x0, int y0, int ax, int by, int p) {
+    const int la0 = x0 == 0 ? 2 : 0;  // staged columns and rows inside the domain
+    const int cols = min(ax + 4, g.na - x0 + 2) - la0;
+    const int lb0 = DIM == 3 && y0 == 0 ? 2 : 0;
+    const int rows = (DIM == 3 ? min(by + 4, g.nb - y0 + 2) : 1) - lb0;
+    const int64_t base = (int64_t)p * g.ps + (DIM == 3 ? (int64_t)(y0 - 2) * g.na : 0) + (x0 - 2);
+    if constexpr (sizeof(R) == 4) {
+      // pairs: every address even (8 bytes), rows of whole pairs
+      const bool pairs = ((g.na | x0 | cols | S.pw) & 1) == 0 &&
+                         ((reinterpret_cast<uintptr_t>(U) | (VARG ? reinterpret_cast<uintptr_t>(gam) : 0)) & 7) == 0;
+      if (pairs) {
+        copy_rows<2>(g, U, gam, dst, S, base, la0, lb0, cols, rows);
+        return;
+      }
+    }
+    copy_rows<1>(g, U, gam, dst, S, base, la0, lb0, cols, rows);
   }
 
   // Stage a plane outside the domain into `dst` by the boundary rules.
