@@ -36,6 +36,8 @@ UNITS = {
     "tfv_host.cu": [],
     "tfv_metric_f64.cu": ["-fmad=false"],
     "tfv_metric_f32.cu": F32,
+    "tfv_metric_tile_f64.cu": ["-fmad=false"],
+    "tfv_metric_tile_f32.cu": F32,
     "tfv_metric_host.cu": [],
 }
 

@@ -94,6 +94,14 @@ struct MArgs {
   double gamma;
   R gam;              // gamma in the arithmetic type
   double dt;          // stage time step
+  // tiled kernels (tfv_metric_tile.cuh): dt formed on the device from the rate
+  // maximum (CFL / rate, limited by the remaining time), 1 / (gamma - 1), tiles
+  // along x and y, per-tile partial sums [tiles][16]
+  int32_t dt_from_rate;
+  double cfl, remaining;
+  R igm1;
+  int32_t ntx, nty;
+  double* tpart;
   int32_t periodic[3];  // face pair of each direction is periodic
   const MFace<R>* face;  // [6] in device memory (x_min, x_max, y_min, ...)
   InstDesc chem;      // chemistry constants (q, ea, a, closure) for react_cell

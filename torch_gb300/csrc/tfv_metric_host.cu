@@ -45,6 +45,11 @@ struct tfv_metric {
   size_t off_state_a = 0, off_q_a[2] = {0, 0}, off_state_b = 0, off_q_b[2] = {0, 0};
   size_t off_p = 0, off_g = 0, off_s = 0, off_k = 0, off_w[3] = {0, 0, 0}, off_t[3] = {0, 0, 0};
   size_t off_faces = 0, off_fac = 0, off_part = 0, off_res = 0, off_rate = 0, off_err = 0, ws_size = 0;
+  // tiled kernels: block, chunk and tile counts;
+  // control block (rate, error words, summed records) and tile records
+  bool tiled = false;
+  int bx = 0, by = 0, chunk = 0, ntx = 0, nty = 0, ntiles = 0;
+  size_t off_ctl = 0, off_tpart = 0;
   unsigned char* ws = nullptr;
   void* ring[2] = {nullptr, nullptr};
   void* lam[2] = {nullptr, nullptr};
@@ -145,7 +150,55 @@ MArgs<R> make_args(const tfv_metric* m) {
   A.part = reinterpret_cast<double*>(m->ws + m->off_part);
   A.rate_max = reinterpret_cast<unsigned long long*>(m->ws + m->off_rate);
   A.err = reinterpret_cast<int32_t*>(m->ws + m->off_err);
+  if (m->tiled) {
+    A.cfl = m->cfg.cfl;
+    A.igm1 = (R)(1.0 / (m->cfg.gamma - 1.0));
+    A.ntx = m->ntx;
+    A.nty = m->nty;
+  }
   return A;
+}
+
+// Block and chunk of the tiled kernels.  A block of bx x by threads updates
+// (bx - 1) x (by - 1) cells (2D: bx - 2); a chunk of c planes costs c + 1.6 (its extra
+// marching face and staged planes).  Single precision: the chunk whose last wave
+// of resident CTAs (two of 256 threads per SM in 3D, four of 128 in 2D) is
+// fullest.  Double precision (2D): 32- or 128-wide blocks by the cost model of
+// the Cartesian tiles (latency per wave of 16 warps plus FP64 pipe time per
+// resident warp).
+void choose_tiles(tfv_metric* m) {
+  const bool d64 = m->esz == 8;
+  const double sms = m->sms;
+  double best = 0.0;
+  static const int kChunks[] = {1, 2, 3, 4, 6, 8, 12, 16, 20, 24, 32, 40, 48, 64};
+  const int widths[2] = {m->dim == 3 ? 16 : 128, 32};
+  for (int k = 0; k < (d64 ? 2 : 1); ++k) {
+    const int bx = widths[k], by = m->dim == 3 ? 16 : 1;
+    const int cells = m->dim == 3 ? bx - 1 : bx - 2;  // along x (MBlock)
+    const int ntx = (m->cfg.n[0] + cells - 1) / cells;
+    const int nty = m->dim == 3 ? (m->cfg.n[1] + by - 2) / (by - 1) : 1;
+    const int np = m->cfg.n[m->dim - 1];
+    for (int c : kChunks) {
+      const double tiles = double(ntx) * nty * ((np + c - 1) / c);
+      double t;
+      if (d64) {
+        const double warps = std::ceil(tiles / sms) * (bx / 32);
+        t = (c + 1.6) * (6.6 * std::ceil(warps / 16.0) + 0.95 * warps);
+      } else {
+        const double slots = sms * (m->dim == 3 ? 2 : 4);
+        t = std::ceil(tiles / slots) * (c + 1.6);
+      }
+      if (best == 0.0 || t < best) {
+        best = t;
+        m->bx = bx;
+        m->by = by;
+        m->chunk = c;
+        m->ntx = ntx;
+        m->nty = nty;
+        m->ntiles = (int)tiles;
+      }
+    }
+  }
 }
 
 int grid_for(const tfv_metric* m, int64_t n) {
@@ -442,6 +495,110 @@ int metric_step(tfv_metric* m) {
   return host_fail(TFV_ENUMERIC, "Could not find a positive metric/face step");
 }
 
+// The step of inert 2D and 3D single-precision sessions through the tiled kernels: rate, both
+// SSPRK2 stages and the reduction of their records are enqueued at once, with
+// dt formed on the device, and the host looks once; dt halvings and
+// first-order retries enqueue the stages again with the host's dt.
+template <typename R>
+int metric_step_tiled(tfv_metric* m) {
+  const tfv_metric_config& c = m->cfg;
+  if (m->time == c.t_end) return TFV_OK;
+  if (m->steps >= c.max_steps)
+    return host_fail(TFV_ENUMERIC, "Maximum steps reached before requested final time");
+  struct Control {
+    unsigned long long rate;
+    int32_t err[4];  // rate, stage 1, stage 2
+    double sums[2][16];
+  };
+  static_assert(sizeof(Control) == 24 + 256, "control block layout");
+  Driver<R> D;
+  D.m = m;
+  D.A = make_args<R>(m);
+  unsigned char* ctl = m->ws + m->off_ctl;
+  double* tpart = reinterpret_cast<double*>(m->ws + m->off_tpart);
+  int32_t* const errs = reinterpret_cast<int32_t*>(ctl + 8);
+  D.A.rate_max = reinterpret_cast<unsigned long long*>(ctl);
+  D.A.remaining = c.t_end - m->time;
+  D.A.chunk = m->chunk;
+  D.s = m->stream;
+  void* const start = m->ring[m->cur];
+  void* const next = m->ring[1 - m->cur];
+  void* const mid = m->ws + m->off_state_b;
+  auto tile = [&](int stage) {
+    return sizeof(R) == 8
+               ? metric_tile_launch_f64(m->dim, m->bx, stage,
+                                        reinterpret_cast<const MArgs<double>&>(D.A), m->ntiles, D.s)
+               : metric_tile_launch_f32(m->dim, m->bx, stage,
+                                        reinterpret_cast<const MArgs<float>&>(D.A), m->ntiles, D.s);
+  };
+  Control h;
+  double dt = 0.0;
+  for (int retry = 0; retry < 20; ++retry) {
+    for (int fo = 0; fo < 2; ++fo) {
+      const bool first = retry == 0 && fo == 0;
+      TFV_MCUDA(cudaMemsetAsync(ctl + (first ? 0 : 8), 0, first ? 24 : 16, D.s));
+      if (first) {
+        D.A.U = (const R*)start;
+        D.A.err = errs;
+        TFV_MCUDA(tile(0));
+      }
+      D.A.dt_from_rate = first;
+      D.A.dt = dt;
+      D.A.first_order = fo;
+      D.A.U = (const R*)start;
+      D.A.Uout = (R*)mid;
+      D.A.err = errs + 1;
+      D.A.tpart = tpart;
+      TFV_MCUDA(tile(1));
+      D.A.U0 = (const R*)start;
+      D.A.U = (const R*)mid;
+      D.A.Uout = (R*)next;
+      D.A.err = errs + 2;
+      D.A.tpart = tpart + (size_t)m->ntiles * 16;
+      TFV_MCUDA(tile(2));
+      TFV_MCUDA(metric_tile_reduce(tpart, m->ntiles, reinterpret_cast<double*>(ctl + 24), D.s));
+      TFV_MCUDA(cudaMemcpyAsync(&h, ctl, sizeof(h), cudaMemcpyDeviceToHost, D.s));
+      TFV_MCUDA(cudaStreamSynchronize(D.s));
+      int r;
+      if (first) {
+        if ((r = D.boundary_error(h.err[0]))) return r;
+        double rate;
+        if (sizeof(R) == 8) {
+          std::memcpy(&rate, &h.rate, sizeof(double));
+        } else {
+          float f;
+          const uint32_t b32 = (uint32_t)h.rate;
+          std::memcpy(&f, &b32, sizeof(float));
+          rate = (double)f;
+        }
+        if (h.err[0] & kMErrRate) rate = NAN;
+        dt = std::min(c.cfl / rate, c.t_end - m->time);
+      }
+      if (fo == 0 && (!std::isfinite(dt) || dt <= 0 || m->time + dt == m->time))
+        return host_fail(TFV_ENUMERIC, "Integration stalled before requested final time");
+      if ((r = D.boundary_error(h.err[1]))) return r;
+      if (h.err[1] & kMErrNonphysical) continue;
+      if ((r = D.boundary_error(h.err[2]))) return r;
+      if (h.err[2] & kMErrNonphysical) continue;
+      // commit (torchSession.py:566-576)
+      for (int v = 0; v < m->nv; ++v) {
+        m->boundary[v] += (0.5 * dt) * (h.sums[0][8 + v] + h.sums[1][8 + v]);
+        m->source[v] += (0.5 * dt) * (h.sums[0][v] + h.sums[1][v]);
+      }
+      m->cur = 1 - m->cur;
+      m->time = std::min(m->time + dt, c.t_end);
+      m->steps += 1;
+      m->dt = dt;
+      m->last_fallback = fo;
+      m->fallback_steps += fo;
+      m->status = m->time == c.t_end ? TFV_DONE : TFV_READY;
+      return TFV_OK;
+    }
+    dt /= 2;  // lost positivity at both orders
+  }
+  return host_fail(TFV_ENUMERIC, "Could not find a positive metric/face step");
+}
+
 template <typename R>
 int upload_faces(tfv_metric* m) {
   MFace<R> faces[6];
@@ -551,6 +708,28 @@ int tfv_metric_create(int32_t precision, const tfv_metric_config* cfg, const dou
   m->off_res = take(sizeof(double) * kSlots * 8);
   m->off_rate = take(sizeof(unsigned long long));
   m->off_err = take(2 * sizeof(int32_t));  // error words of the two SSPRK2 stages
+  {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&m->sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+      cudaGetLastError();
+      m->sms = 152;  // no device here: the workspace is only sized
+    }
+  }
+  // Inert sessions run the tiled kernels, whose stage reads and writes the state
+  // once.  Not double precision in 3D: it is bound by the FP64 pipe, and there
+  // the slopes of the halo and the marching faces at chunk edges, which the tiled
+  // kernels form twice, cost more than the passes they save.  Step times, tiled
+  // against separate kernels: 3D fp64 64 x 48 x 48 1101 / 731 us, 128 x 96 x 96
+  // 4794 / 3567 us; 2D fp64 40 x 36 119 / 231 us, 256 x 192 168 / 259 us, 1024 x
+  // 768 1212 / 1204 us; 3D fp32 16 x 12 x 12 70 / 226 us, 256 x 192 x 192 1325 /
+  // 2020 us; 2D fp32 2048 x 1024 187 / 458 us.
+  m->tiled = (m->dim == 2 || (m->dim == 3 && m->esz == 4)) && m->nfrac == 0 && m->nc < (int64_t(1) << 31);
+  if (m->tiled) {
+    choose_tiles(m);
+    m->off_ctl = take(24 + 2 * 16 * sizeof(double));
+    m->off_tpart = take(sizeof(double) * 2 * 16 * m->ntiles);
+  }
   m->ws_size = o;
   *out = m;
   return TFV_OK;
@@ -614,7 +793,10 @@ int tfv_metric_bind(tfv_metric* m, void* workspace, void* const* states, void* c
 int tfv_metric_advance(tfv_metric* m, int32_t nsteps) {
   if (!m || !m->bound) return host_fail(TFV_EINVAL, "session not bound");
   for (int32_t k = 0; k < nsteps && m->time != m->cfg.t_end; ++k) {
-    const int r = m->precision == TFV_FP64 ? metric_step<double>(m) : metric_step<float>(m);
+    const int r = m->tiled ? (m->precision == TFV_FP64 ? metric_step_tiled<double>(m)
+                                                       : metric_step_tiled<float>(m))
+                           : (m->precision == TFV_FP64 ? metric_step<double>(m)
+                                                       : metric_step<float>(m));
     if (r) return r;
   }
   return TFV_OK;

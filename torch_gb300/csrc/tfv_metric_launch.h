@@ -23,6 +23,14 @@ cudaError_t metric_launch_f64(int op, int dim, const MArgs<double>& A, int arg, 
                               int block, cudaStream_t s);
 cudaError_t metric_launch_f32(int op, int dim, const MArgs<float>& A, int arg, int grid,
                               int block, cudaStream_t s);
+// tiled kernels of inert 2D / 3D sessions: stage 0 the CFL rate, 1 and 2 the
+// SSPRK2 stages; bx: block width of 2D grids (32 or 128)
+cudaError_t metric_tile_launch_f64(int dim, int bx, int stage, const MArgs<double>& A, int grid,
+                                   cudaStream_t s);
+cudaError_t metric_tile_launch_f32(int dim, int bx, int stage, const MArgs<float>& A, int grid,
+                                   cudaStream_t s);
+// out[2][16] = sums of part[2][ntiles][16] over the tiles
+cudaError_t metric_tile_reduce(const double* part, int ntiles, double* out, cudaStream_t s);
 // Rusanov fluxes of n faces (rows [nv][n], primitive face states)
 cudaError_t rusanov_launch_f64(int nv, int64_t n, int dir, const void* l, const void* r,
                                const void* gl, const void* gr, void* out, int grid,
