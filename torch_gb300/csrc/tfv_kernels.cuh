@@ -583,7 +583,11 @@ __device__ __forceinline__ void cell_stage(const R* ringm, const R* ringc, const
       vp[c] = u[c] + half_slope(s[c]);
       vm[c] = u[c] - half_slope(s[c]);
     }
-    if (DIM == 3) {
+    if constexpr (!Exact<R>::value && DIM == 3) {
+      flux3_pair(vp, vm, g, dd + 1, fp, fm);
+    } else if constexpr (!Exact<R>::value) {
+      flux2_pair(vp, vm, g, dd, fp, fm);
+    } else if (DIM == 3) {
       flux3<R>(vp, g, dd + 1, fp);
       flux3<R>(vm, g, dd + 1, fm);
     } else {

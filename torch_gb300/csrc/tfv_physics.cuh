@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tfv_pair.cuh"
 #include "tfv_soft64.cuh"
 
 namespace tfv {
@@ -240,6 +241,26 @@ __device__ __forceinline__ void flux3(const R* u, R g, int m, R* f) {
   f[4] = vel * (u[4] + p);
 }
 
+// flux3 of two states in packed arithmetic, single precision.
+__device__ __forceinline__ void flux3_pair(const float* ua, const float* ub, float g, int m,
+                                           float* fa, float* fb) {
+  Pair u[5];
+#pragma unroll
+  for (int c = 0; c < 5; ++c) u[c] = pk(ua[c], ub[c]);
+  const Pair ssum = fma2(u[3], u[3], fma2(u[2], u[2], u[1] * u[1]));
+  const Pair ir = pk(rcp(ua[0]), rcp(ub[0]));
+  const Pair p = pk(g - 1.0f) * fma2(ssum * ir, pk(-0.5f), u[4]);
+  const Pair vel = u[m] * ir;
+  fa[0] = ua[m];
+  fb[0] = ub[m];
+#pragma unroll
+  for (int c = 1; c < 4; ++c) {
+    const Pair f = c == m ? fma2(u[c], vel, p) : u[c] * vel;
+    unpk(f, fa[c], fb[c]);
+  }
+  unpk(vel * (u[4] + p), fa[4], fb[4]);
+}
+
 template <typename R>
 __device__ __forceinline__ void flux2(const R* u, R g, int normal, R* f) {
   const R rho = floored(u[0]);
@@ -265,6 +286,29 @@ __device__ __forceinline__ void flux2(const R* u, R g, int normal, R* f) {
     f[2] = rho * (vy * vy) + p;
     f[3] = vy * (u[3] + p);
   }
+}
+
+// flux2 of two states in packed arithmetic, single precision.
+__device__ __forceinline__ void flux2_pair(const float* ua, const float* ub, float g, int normal,
+                                           float* fa, float* fb) {
+  const float ra = floored(ua[0]), rb = floored(ub[0]);
+  const Pair r = pk(ra, rb), ir = pk(rcp(ra), rcp(rb)), e = pk(ua[3], ub[3]);
+  const Pair vx = pk(ua[1], ub[1]) * ir, vy = pk(ua[2], ub[2]) * ir;
+  const Pair pe = pk(g - 1.0f) * fma2(r * pk(-0.5f), fma2(vy, vy, vx * vx), e);
+  const Pair p = pk(floored(lo_(pe)), floored(hi_(pe)));
+  const Pair vn = normal == 0 ? vx : vy;
+  const Pair mx = r * vx;
+  if (normal == 0) {
+    unpk(mx, fa[0], fb[0]);
+    unpk(fma2(mx, vx, p), fa[1], fb[1]);
+    unpk(mx * vy, fa[2], fb[2]);
+  } else {
+    const Pair my = r * vy;
+    unpk(my, fa[0], fb[0]);
+    unpk(mx * vy, fa[1], fb[1]);
+    unpk(fma2(my, vy, p), fa[2], fb[2]);
+  }
+  unpk(vn * (e + p), fa[3], fb[3]);
 }
 
 // Physical-state test of one cell (python/cfdSolver/torchSolver.py:1038-1046).
@@ -397,68 +441,59 @@ __device__ __forceinline__ void hllc_f32(const float* ul, const float* ur, float
   using R = float;
   constexpr int NV = NT + 3;
   constexpr int E = NV - 1;
+  // the two sides are the halves of packed pairs
   const R g = R(0.5) * (gl + gr);
   const R rl = np_max(ul[0], R(kFloor));
   const R rr = np_max(ur[0], R(kFloor));
   const R irl = rcp(rl), irr = rcp(rr);
-  const R unl = ul[1] * irl;
-  const R unr = ur[1] * irr;
+  const Pair r = pk(rl, rr), ir = pk(irl, irr), e = pk(ul[E], ur[E]);
+  const Pair un2 = pk(ul[1], ur[1]) * ir;
+  Pair ut[NT];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) ut[t] = pk(ul[2 + t], ur[2 + t]) * ir;
+  Pair q = ut[0] * ut[0];
+#pragma unroll
+  for (int t = 1; t < NT; ++t) q = fma2(ut[t], ut[t], q);
+  q = fma2(un2, un2, q);
+  const Pair ei = fma2(r * pk(-0.5f), q, e);  // internal energy density
+  const R pl = np_max((gl - R(1)) * lo_(ei), R(kFloor));
+  const R pr = np_max((gr - R(1)) * hi_(ei), R(kFloor));
+  const Pair p2 = pk(pl, pr);
+  const Pair a2 = (pk(gl, gr) * p2) * ir;
+  const R al = sqrtf(lo_(a2)), ar = sqrtf(hi_(a2));
+  const Pair ep = e + p2;
+
+  const Pair mn = r * un2;
+  R fl[NV], fr[NV];
+  unpk(mn, fl[0], fr[0]);
+  unpk(fma2(mn, un2, p2), fl[1], fr[1]);
+#pragma unroll
+  for (int t = 0; t < NT; ++t) unpk(mn * ut[t], fl[2 + t], fr[2 + t]);
+  unpk(un2 * ep, fl[E], fr[E]);
+
+  const R sql = sqrtf(rl), sqr = sqrtf(rr);
+  const R inv = rcp(sql + sqr);
+  const R wl = sql * inv, wr = sqr * inv;  // Roe weights
+  const R unl = lo_(un2), unr = hi_(un2);
   R utl[NT], utr[NT];
 #pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    utl[t] = ul[2 + t] * irl;
-    utr[t] = ur[2 + t] * irr;
-  }
-  R stl = utl[0] * utl[0], str = utr[0] * utr[0];
-#pragma unroll
-  for (int t = 1; t < NT; ++t) {
-    stl = stl + utl[t] * utl[t];
-    str = str + utr[t] * utr[t];
-  }
-  const R kel = (R(0.5) * rl) * (unl * unl + stl);
-  const R ker = (R(0.5) * rr) * (unr * unr + str);
-  const R pl = np_max((gl - R(1)) * (ul[E] - kel), R(kFloor));
-  const R pr = np_max((gr - R(1)) * (ur[E] - ker), R(kFloor));
-  const R al = sqrt(gl * pl * irl);
-  const R ar = sqrt(gr * pr * irr);
-
-  R fl[NV], fr[NV];
-  fl[0] = rl * unl;
-  fl[1] = rl * (unl * unl) + pl;
-  fr[0] = rr * unr;
-  fr[1] = rr * (unr * unr) + pr;
+  for (int t = 0; t < NT; ++t) unpk(ut[t], utl[t], utr[t]);
+  const R uroe = wl * unl + wr * unr;
+  R vsum = uroe * uroe;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {
-    fl[2 + t] = (rl * unl) * utl[t];
-    fr[2 + t] = (rr * unr) * utr[t];
+    const R vt = wl * utl[t] + wr * utr[t];
+    vsum = vsum + vt * vt;
   }
-  fl[E] = unl * (ul[E] + pl);
-  fr[E] = unr * (ur[E] + pr);
-
-  const R sql = sqrt(rl);
-  const R sqr = sqrt(rr);
-  const R inv = rcp(sql + sqr);
-  const R uroe = (sql * unl + sqr * unr) * inv;
-  R vsum;
-  {
-    const R v0 = (sql * utl[0] + sqr * utr[0]) * inv;
-    vsum = v0 * v0;
-#pragma unroll
-    for (int t = 1; t < NT; ++t) {
-      const R vt = (sql * utl[t] + sqr * utr[t]) * inv;
-      vsum = vsum + vt * vt;
-    }
-  }
-  const R hl = (ul[E] + pl) * irl;
-  const R hr = (ur[E] + pr) * irr;
-  const R hroe = (sql * hl + sqr * hr) * inv;
-  const R keroe = R(0.5) * (uroe * uroe + vsum);
-  const R aroe = sqrt(np_max((g - R(1)) * (hroe - keroe), R(kFloor)));
+  const Pair h = ep * ir;
+  const R hroe = wl * lo_(h) + wr * hi_(h);
+  const R aroe = sqrtf(np_max((g - R(1)) * (hroe - R(0.5) * vsum), R(kFloor)));
 
   const R sL = np_min(unl - al, uroe - aroe);
   const R sR = np_max(unr + ar, uroe + aroe);
-  const R den = guarded(rl * (sL - unl) - rr * (sR - unr), R(kGuard));
-  const R ss = dv(((pr - pl) + (rl * unl) * (sL - unl)) - (rr * unr) * (sR - unr), den);
+  const Pair m = r * (pk(sL, sR) - un2);
+  const R den = guarded(lo_(m) - hi_(m), R(kGuard));
+  const R ss = dv(((pr - pl) + unl * lo_(m)) - unr * hi_(m), den);
 
   // star state of the side whose star region can be selected
   const bool right = (ss <= R(0));
@@ -532,83 +567,79 @@ __device__ __forceinline__ void hllc_gated(const float* ul, const float* ur, flo
   constexpr int E = NV - 1;
   const float fl = float(kFloor);
   const float g = 0.5f * (gl + gr);
-  // the density floors of the reference change nothing here: a face state
+  // the two sides are the halves of packed pairs up to the wave speeds.  The
+  // density floors of the reference change nothing here: a face state
   // whose density is not above the floor fails the gate test below and the
   // step is redone to first order
-  const float rl = ul[0];
-  const float rr = ur[0];
-  const float irl = rcp(rl), irr = rcp(rr);
-  const float unl = ul[1] * irl, unr = ur[1] * irr;
-  float utl[NT], utr[NT];
+  const Pair r = pk(ul[0], ur[0]), e = pk(ul[E], ur[E]);
+  const float irl = rcp(ul[0]), irr = rcp(ur[0]);
+  const Pair ir = pk(irl, irr);
+  const Pair un = pk(ul[1], ur[1]) * ir;
+  Pair ut[NT];
 #pragma unroll
-  for (int t = 0; t < NT; ++t) {
-    utl[t] = ul[2 + t] * irl;
-    utr[t] = ur[2 + t] * irr;
-  }
-  float stl = utl[0] * utl[0], str = utr[0] * utr[0];
+  for (int t = 0; t < NT; ++t) ut[t] = pk(ul[2 + t], ur[2 + t]) * ir;
+  Pair q = ut[0] * ut[0];
 #pragma unroll
-  for (int t = 1; t < NT; ++t) {
-    stl = stl + utl[t] * utl[t];
-    str = str + utr[t] * utr[t];
-  }
-  const float eil = ul[E] - (0.5f * rl) * (unl * unl + stl);  // internal energy density
-  const float eir = ur[E] - (0.5f * rr) * (unr * unr + str);
+  for (int t = 1; t < NT; ++t) q = fma2(ut[t], ut[t], q);
+  q = fma2(un, un, q);
+  const Pair ei = fma2(r * pk(-0.5f), q, e);  // internal energy density
+  float eil, eir;
+  unpk(ei, eil, eir);
   if (!(ul[0] > fl && eil > fl && ur[0] > fl && eir > fl)) gate = true;
   const float pl = np_max((gl - 1.0f) * eil, fl);
   const float pr = np_max((gr - 1.0f) * eir, fl);
-  const float al = sqrtf(gl * pl * irl);
-  const float ar = sqrtf(gr * pr * irr);
-  const float sql = sqrtf(rl), sqr = sqrtf(rr);
+  const Pair p2 = pk(pl, pr);
+  const Pair a2 = (pk(gl, gr) * p2) * ir;
+  const float al = sqrtf(lo_(a2)), ar = sqrtf(hi_(a2));
+  const float sql = sqrtf(ul[0]), sqr = sqrtf(ur[0]);
   const float inv = rcp(sql + sqr);
-  const float uroe = (sql * unl + sqr * unr) * inv;
-  float vsum;
-  {
-    const float v0 = (sql * utl[0] + sqr * utr[0]) * inv;
-    vsum = v0 * v0;
+  const float wl = sql * inv, wr = sqr * inv;  // Roe weights
+  const float unl = lo_(un), unr = hi_(un);
+  const float uroe = wl * unl + wr * unr;
+  float vsum = uroe * uroe;
 #pragma unroll
-    for (int t = 1; t < NT; ++t) {
-      const float vt = (sql * utl[t] + sqr * utr[t]) * inv;
-      vsum = vsum + vt * vt;
-    }
+  for (int t = 0; t < NT; ++t) {
+    const float vt = wl * lo_(ut[t]) + wr * hi_(ut[t]);
+    vsum = vsum + vt * vt;
   }
-  const float hl = (ul[E] + pl) * irl;
-  const float hr = (ur[E] + pr) * irr;
-  const float hroe = (sql * hl + sqr * hr) * inv;
-  const float aroe = sqrtf(np_max((g - 1.0f) * (hroe - 0.5f * (uroe * uroe + vsum)), fl));
+  const Pair h = (e + p2) * ir;
+  const float hroe = wl * lo_(h) + wr * hi_(h);
+  const float aroe = sqrtf(np_max((g - 1.0f) * (hroe - 0.5f * vsum), fl));
   const float sL = np_min(unl - al, uroe - aroe);
   const float sR = np_max(unr + ar, uroe + aroe);
-  const float den = guarded(rl * (sL - unl) - rr * (sR - unr), float(kGuard));
-  const float ss = dv(((pr - pl) + (rl * unl) * (sL - unl)) - (rr * unr) * (sR - unr), den);
+  const Pair gap = pk(sL, sR) - un;
+  const Pair m = r * gap;
+  const float ml_ = lo_(m), mr_ = hi_(m);
+  const float den = guarded(ml_ - mr_, float(kGuard));
+  const float ss = dv(((pr - pl) + unl * ml_) - unr * mr_, den);
 
   const bool mr = (0.0f >= sR);
   const bool mstar = ((ss <= 0.0f) && (0.0f <= sR)) || ((sL <= 0.0f) && (0.0f <= ss));
   const bool ml = (0.0f <= sL);
   // side whose flux the selected region reads
   const bool right = mr || (mstar && ss <= 0.0f);
-  const float rho = right ? rr : rl;
   const float irho = right ? irr : irl;
-  const float un = right ? unr : unl;
+  const float v = right ? unr : unl;
   const float p = right ? pr : pl;
-  const float uE = right ? ur[E] : ul[E];
   float u[NV], f[NV];
 #pragma unroll
   for (int c = 0; c < NV; ++c) u[c] = right ? ur[c] : ul[c];
-  const float mn = rho * un;
-  f[0] = mn;
-  f[1] = mn * un + p;
+  f[0] = u[1];  // rho * (m / rho) is the momentum itself
+  f[1] = u[1] * v + p;
 #pragma unroll
-  for (int t = 0; t < NT; ++t) f[2 + t] = mn * (right ? utr[t] : utl[t]);
-  f[E] = un * (uE + p);
+  for (int t = 0; t < NT; ++t) f[2 + t] = u[2 + t] * v;
+  f[E] = v * (u[E] + p);
   const float s = right ? sR : sL;
   if (!mr && mstar && !(fabsf(s - ss) < fl)) {
-    const float rho_s = np_max(rho * dv(s - un, guarded(s - ss, float(kGuard))), fl);
-    const float dun = guarded(s - un, float(kGuard));
+    const float rho_s = np_max(u[0] * dv(s - v, guarded(s - ss, float(kGuard))), fl);
+    const float dun = guarded(s - v, float(kGuard));
+    const float k = rho_s * irho;  // star to side density
     float star[NV];
     star[0] = rho_s;
     star[1] = rho_s * ss;
 #pragma unroll
-    for (int t = 0; t < NT; ++t) star[2 + t] = rho_s * (right ? utr[t] : utl[t]);
-    star[E] = rho_s * (uE * irho + (ss - un) * (ss + dv(p, rho * dun)));
+    for (int t = 0; t < NT; ++t) star[2 + t] = k * u[2 + t];
+    star[E] = k * u[E] + (rho_s * (ss - v)) * (ss + dv(p, u[0] * dun));
 #pragma unroll
     for (int c = 0; c < NV; ++c) f[c] = f[c] + s * (star[c] - u[c]);
   }
