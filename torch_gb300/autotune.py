@@ -27,14 +27,16 @@ def candidates(dim, precision, sms):
     if dim == 3:
         shapes = [(16, 16), (32, 8)] if precision == "fp32" else [(32, 4), (16, 8)]
         for tx, ty in shapes:
-            for chunk in (16, 32, 40, 64):
+            # short chunks give small grids enough tiles (single precision's default
+            # picks them the same way)
+            for chunk in (3, 8, 16, 32, 40, 64):
                 out.append((tx, ty, chunk, 0, 1))
     elif dim == 2:
         # 124: rows of 124 cells whose two ring cells take the lanes after the
         # owners (single precision only: double precision tiles are whole warps)
         for tx in ((124, 128, 256) if precision == "fp32" else (128, 256)):
-            for chunk in (16, 32, 64):
-                for pers in (0, 2 * sms):
+            for chunk in (2, 6, 16, 32, 64):
+                for pers in (0, 2 * sms) if chunk >= 16 else (0,):
                     out.append((tx, 1, chunk, pers, 1))
     else:
         for tx in (128, 256):

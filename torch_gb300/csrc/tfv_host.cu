@@ -735,13 +735,55 @@ static void fp64_tile(tfv_batch* b, const tfv_config* cfgs) {
   }
 }
 
+// Planes per chunk of the single-precision default tiles: the longest chunk
+// (the caller's) where the batch fills the chip with it, shorter ones where
+// that leaves SMs idle.  A chunk of c planes costs c + 3.5 plane times (two more
+// cell stages, prologue and epilogue); a plane takes a + b k microseconds with
+// k tiles resident on the SM, fitted on the GB300 (2D: a 1.64, b 0.264, up to 8;
+// 3D: 4.05, 0.55, up to 3).  Measured step times, longest chunk against the
+// chosen one: 3D 32^3 121 / 51 us (1 plane), 64^3 137 / 70 (3), 96^3 148 / 114
+// (8); 2D 64^2 49 / 22 us (1), 256^2 51 / 29 (2), 512^2 56 / 37 (3).  From 10%
+// of predicted gain on: where the chip is full the chunks are alike in the
+// model, and the longest is the fastest measured (256^3 959 us with 40 planes,
+// 997 with 32).
+static int fp32_chunk(const tfv_batch* b, const tfv_config* cfgs, int tx, int ty, int longest) {
+  const bool d3 = b->dim == 3;
+  const double sms = device_sms();
+  const double a = d3 ? 4.05 : 1.64, bk = d3 ? 0.55 : 0.264, resident = d3 ? 3 : 8;
+  auto cost = [&](int c) {
+    double tiles = 0.0, work = 0.0, longest_tile = 0.0;
+    for (int i = 0; i < b->n; ++i) {
+      const int32_t* n = cfgs[i].counts;
+      const double planes = n[d3 ? 2 : 1], chunks = std::ceil(planes / c);
+      const double columns = std::ceil(double(n[0]) / tx) * (d3 ? std::ceil(double(n[1]) / ty) : 1.0);
+      const double area = 0.3 * columns + 0.7 * (double(n[0]) / tx) * (d3 ? double(n[1]) / ty : 1.0);
+      tiles += columns * chunks;
+      work += area * (planes + 3.5 * chunks);
+      longest_tile = std::max(longest_tile, std::min<double>(c, planes) + 3.5);
+    }
+    const double slots = sms * resident;
+    if (tiles <= slots) return longest_tile * (a + bk * std::ceil(tiles / sms));
+    return (work / slots + 0.5 * longest_tile) * (a + bk * resident);
+  };
+  int best = longest;
+  double t = 0.9 * cost(longest);
+  for (int c = 1; c < longest; ++c) {
+    const double tc = cost(c);
+    if (tc < t) {
+      t = tc;
+      best = c;
+    }
+  }
+  return best;
+}
+
 static void default_tile(tfv_batch* b, const tfv_config* cfgs) {
   // FP32 3D: 16 x 16 (three CTAs per SM; the fastest measured shape at 256^3),
-  // 40-plane chunks (256^3: 1.065 ms per step kernel against 1.105 with 32 and
+  // chunks of at most 40 planes (256^3: 1.065 ms per step kernel against 1.105 with 32 and
   // 1.085 with 48, measured).
   // FP32 2D: rows of 124 cells in 128 threads (the two ring cells on the
-  // spare lanes: no warp does a second cell stage or face per row), 32-row
-  // chunks (4096^2: 31.9 G cell-updates/s against 29.8 for 128 x 32; 64-row
+  // spare lanes: no warp does a second cell stage or face per row), chunks of at
+  // most 32 rows (4096^2: 31.9 G cell-updates/s against 29.8 for 128 x 32; 64-row
   // chunks reach 32.5 there but leave small grids too few tiles: the
   // autotuner tries them per batch).
   b->tile.persistent_ctas = 0;
@@ -759,9 +801,10 @@ static void default_tile(tfv_batch* b, const tfv_config* cfgs) {
     fp64_tile(b, cfgs);
   } else if (b->dim == 3) {
     b->tile.tx = b->tile.ty = 16;
-    b->tile.chunk = 40;
+    b->tile.chunk = fp32_chunk(b, cfgs, 16, 16, 40);
   } else {
     b->tile.tx = 124;
+    b->tile.chunk = fp32_chunk(b, cfgs, 124, 1, 32);
   }
 }
 
