@@ -174,12 +174,18 @@ int resident_slots(const tfv_batch* b) {
 
 // Completion time of `dur` dispatched in order onto `slots` resident CTAs
 // (each block starts on the first slot that frees up).
+// The first `slots` blocks start at once; a launch that fits needs no heap (a
+// 192^2 double-precision step function spent 200 of its 745 us here).
 double dispatch_makespan(const std::vector<double>& dur, int slots) {
-  std::vector<double> heap(static_cast<size_t>(slots), 0.0);
+  const size_t first = std::min(dur.size(), static_cast<size_t>(slots));
+  std::vector<double> heap(dur.begin(), dur.begin() + first);
   double end = 0.0;
-  for (double d : dur) {
+  for (double d : heap) end = std::max(end, d);
+  if (first == dur.size()) return end;
+  std::make_heap(heap.begin(), heap.end(), std::greater<double>());
+  for (size_t k = first; k < dur.size(); ++k) {
     std::pop_heap(heap.begin(), heap.end(), std::greater<double>());
-    heap.back() += d;
+    heap.back() += dur[k];
     end = std::max(end, heap.back());
     std::push_heap(heap.begin(), heap.end(), std::greater<double>());
   }

@@ -28,8 +28,11 @@ def _device():
 
 
 def _as_device(x, dtype, device):
-    return torch.as_tensor(np.array(x, copy=True) if isinstance(x, np.ndarray) else x,
-                           dtype=dtype, device=device).contiguous()
+    # the transfer to the device copies a plain array; others (reversed, read-only,
+    # strided) become one first
+    if isinstance(x, np.ndarray) and not (x.flags.c_contiguous and x.flags.writeable):
+        x = np.array(x, copy=True)
+    return torch.as_tensor(x, dtype=dtype, device=device).contiguous()
 
 
 def _out(t, host):
