@@ -105,7 +105,7 @@ typedef struct tfv_tile {
   int32_t chunk;   /* planes marched per tile (z in 3D, y in 2D) */
   int32_t persistent_ctas; /* 0 = one CTA per tile, else grid size of a persistent launch */
   int32_t tma;     /* 1: stage planes with tensor copies (cp.async.bulk.tensor) where the
-                      grid allows it (x extent a multiple of 16 bytes); 0: plain loads */
+                      grid allows it (x extent a multiple of 16 bytes); 0: element copies */
 } tfv_tile;
 
 /* Per-instance scalars read back after steps. */
@@ -226,9 +226,10 @@ int tfv_hydro_step(const tfv_config* cfg, int32_t precision, const void* state_i
  * The step's scratch (descriptors, tile table, per-tile partial sums, and
  * per-cell interface data of 1D tubes) lives in a 1 MiB array inside the
  * library's device image; every GPU that loads the library holds it until the
- * process exits.  Grids whose scratch would not fit are rejected with
- * TFV_EINVAL; tfv_step_workspace_size gives a grid's need (with the default
- * tiles a 3D 256^3 grid needs about 376 KiB in fp32 and 856 KiB in fp64, so
+ * process exits.  A grid whose default tiles need more (tfv_step_workspace_size)
+ * takes the largest tiles instead; grids whose scratch would not fit even so
+ * are rejected with TFV_EINVAL (a 3D 256^3 grid needs about 376 KiB in fp32 and
+ * 856 KiB in fp64 with the largest tiles, so
  * fp64 3D grids much larger than 256^3 are rejected; a 2D 4096^2 grid needs
  * 456 KiB in fp32 and 856 KiB in fp64; 1D tubes need about 49 B per cell in
  * fp32 and 97 B in fp64, so tubes beyond about 21,000 / 10,800 cells are

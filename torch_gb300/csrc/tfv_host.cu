@@ -785,13 +785,12 @@ static int fp32_chunk(const tfv_batch* b, const tfv_config* cfgs, int tx, int ty
 
 static void default_tile(tfv_batch* b, const tfv_config* cfgs) {
   // FP32 3D: 16 x 16 (three CTAs per SM; the fastest measured shape at 256^3),
-  // chunks of at most 40 planes (256^3: 1.065 ms per step kernel against 1.105 with 32 and
-  // 1.085 with 48, measured).
+  // chunks of at most 40 planes (256^3: 0.959 ms per step against 0.996 with 32
+  // and 0.970 with 48).
   // FP32 2D: rows of 124 cells in 128 threads (the two ring cells on the
   // spare lanes: no warp does a second cell stage or face per row), chunks of at
-  // most 32 rows (4096^2: 31.9 G cell-updates/s against 29.8 for 128 x 32; 64-row
-  // chunks reach 32.5 there but leave small grids too few tiles: the
-  // autotuner tries them per batch).
+  // most 32 rows (4096^2: 492 us per step, 489 with 48 and 536 with 64; 128-cell rows
+  // were 7% slower).
   b->tile.persistent_ctas = 0;
   b->tile.tma = 1;
   b->tile.ty = 1;
