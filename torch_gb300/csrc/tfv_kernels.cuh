@@ -520,7 +520,7 @@ struct HydroTile {
 __device__ __forceinline__ double half_slope(double s) { return s; }
 __device__ __forceinline__ float half_slope(float s) { return 0.5f * s; }
 
-// Cell stage at local position (a, b) of the current plane: limited slopes in
+// Cell stage of the cell at ring index li and box index bi: limited slopes in
 // every direction and the Hancock predictor (python/cfdSolver/torchSolver3D.py:
 // 135-151, python/cfdSolver/torchSolver2D.py:305-377).  Writes predictor and
 // in-plane slopes to the box; returns the marching-axis slope; sets *gate when
@@ -531,13 +531,11 @@ __device__ __forceinline__ float half_slope(float s) { return 0.5f * s; }
 // face states no face consumes.
 template <typename R, int DIM, bool VARG, int LIM>
 __device__ __forceinline__ void cell_stage(const R* ringm, const R* ringc, const R* ringp,
-                                           R* box, const HydroSmem<R, DIM, VARG>& S, int a,
-                                           int b, R gconst, const R* coefh, R* ubar, R* smarch,
+                                           R* box, const HydroSmem<R, DIM, VARG>& S, int li,
+                                           int bi, R gconst, const R* coefh, R* ubar, R* smarch,
                                            bool& gate, bool check_gate = true) {
   constexpr int NV = DIM + 2;
   const int plane = S.ph * S.pw;
-  const int li = (DIM == 3 ? (b + 2) * S.pw : 0) + (a + S.xo);
-  const int bi = (DIM == 3 ? (b + 1) * S.bw : 0) + (a + 1);
   const int bplane = S.bh * S.bw;
   R* bub = box;                   // predictor
   R* bsa = box + NV * bplane;     // slope along a (x)
@@ -856,8 +854,12 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
   }
 
   // Per-thread work items, computed once per tile and kept in shared memory:
-  // ring/corner cells of the cross region and in-plane faces, packed as
-  // (kind << 30) | ((i + 1) << 15) | (j + 1).
+  // ring / corner cells of the cross region, packed as ((a + 1) << 15) | (b + 1),
+  // and in-plane faces as the indexes that each plane reads, (normal to y << 31) |
+  // (left cell's box << 16) | flux slot (positions decoded per plane took some
+  // fifteen integer instructions a face: 32 2D grids 464 -> 451 us per step, six
+  // 3D grids 866 -> 863, 256^3 unchanged; the ring cells' indexes packed the same
+  // way spilled more, 256^3 965 -> 986).
   int* items = smem_at<int>(smem, S.items_off);
   const int NT = blockDim.x;
   constexpr int MR = HydroSmem<R, DIM, VARG>::kMaxRingItems;
@@ -895,17 +897,18 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
   // the owners they start at thread 0
   const int tface = r0 ? tid : (tid + NT - 64 % NT) % NT;
   for (int w = tface; w < nfa + nfb; w += NT) {
-    int packed;
+    unsigned packed;
     if (w < nfa) {
       const int af = w % (ax + 1), b = w / (ax + 1);
-      packed = ((af + 1) << 15) | (b + 1);
+      packed = ((unsigned)((DIM == 3 ? (b + 1) * S.bw : 0) + af) << 16) |
+               (unsigned)(b * (S.tx + 1) + af);
     } else {
       const int q = w - nfa;
       const int a = q % ax, bf = q / ax;
-      packed = (1 << 30) | ((a + 1) << 15) | (bf + 1);
+      packed = 0x80000000u | ((unsigned)(bf * S.bw + a + 1) << 16) | (unsigned)(bf * S.tx + a);
     }
     if (!TFV_IN(20, n_fitems, (HydroSmem<R, DIM, VARG>::kMaxFaceItems))) break;
-    items[(MR + n_fitems) * NT + tid] = packed;
+    items[(MR + n_fitems) * NT + tid] = (int)packed;
     ++n_fitems;
   }
 
@@ -927,12 +930,12 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
         a = ((pk >> 15) & 0x7fff) - 1;
         b = (pk & 0x7fff) - 1;
       }
-      R ub[NV], sm[NV];
-      // ghost cells (outside the domain) keep the explicit gate; the face
-      // states of in-domain cells are gated where HLLC consumes them (FP32)
+      const int li = (DIM == 3 ? (b + 2) * S.pw : 0) + (a + S.xo);
+      const int bi = (DIM == 3 ? (b + 1) * S.bw : 0) + (a + 1);
       const bool ghost = it < 0 || it >= g.np || x0 + a < 0 || x0 + a >= g.na ||
                          (DIM == 3 && (y0 + b < 0 || y0 + b >= g.nb));
-      cell_stage<R, DIM, VARG, LIM>(rm, rc, rp, box, S, a, b, gconst, coefh, ub, sm, gate,
+      R ub[NV], sm[NV];
+      cell_stage<R, DIM, VARG, LIM>(rm, rc, rp, box, S, li, bi, gconst, coefh, ub, sm, gate,
                                     Exact<R>::value || ghost);
       if (k < 0) {
 #pragma unroll
@@ -948,12 +951,11 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
     if (full) {
       const R* bub = box;
       for (int k = 0; k < n_fitems; ++k) {
-        const int pk = items[(MR + k) * NT + tid];
-        const int kind = pk >> 30;  // 0: face normal to x, 1: normal to y (3D)
-        const int i = ((pk >> 15) & 0x7fff) - 1;
-        const int j = (pk & 0x7fff) - 1;
+        const int item = items[(MR + k) * NT + tid];
+        const int kind = DIM == 3 && item < 0 ? 1 : 0;  // 0: face normal to x, 1: normal to y (3D)
+        const int fo = item & 0xffff;                   // its flux slot
         // left cell's box index, step to the right cell, slope array
-        const int bl = kind == 0 ? (DIM == 3 ? (j + 1) * S.bw : 0) + i : j * S.bw + i + 1;
+        const int bl = (item >> 16) & 0x7fff;
         const int br = bl + (kind == 0 ? 1 : S.bw);
         if (!TFV_IN(21, bl, bplane) || !TFV_IN(22, br, bplane)) continue;
         const R* bsl = box + (kind == 0 ? 1 : 2) * NV * bplane;
@@ -966,9 +968,9 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
           ur[c] = bub[cc * bplane + br] - half_slope(bsl[cc * bplane + br]);
         }
         R gl = gconst, gr = gconst;
-        if (VARG) {
-          const int li = kind == 0 ? (DIM == 3 ? (j + 2) * S.pw : 0) + i - 1 + S.xo
-                                   : (j + 1) * S.pw + i + S.xo;
+        if (VARG) {  // box row r, column q is ring row r + 1, column q - 1 + xo
+          const int r = DIM == 3 ? bl / S.bw : 0;
+          const int li = (DIM == 3 ? (r + 1) * S.pw : 0) + (bl - r * S.bw) - 1 + S.xo;
           gl = rc[S.goff + li];
           gr = rc[S.goff + li + (kind == 0 ? 1 : S.pw)];
         }
@@ -980,22 +982,22 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
 #pragma unroll
         for (int c = 0; c < NV; ++c) F[c] = kind == 1 ? (c == 1 ? f[2] : (c == 2 ? f[1] : f[c])) : f[c];
         if (kind == 0) {
-          const int af = i, b = j;
 #pragma unroll
           for (int c = 0; c < NV; ++c)
-            if (TFV_IN(23, b * (S.tx + 1) + af, fa_plane)) fa[c * fa_plane + b * (S.tx + 1) + af] = F[c];
+            if (TFV_IN(23, fo, fa_plane)) fa[c * fa_plane + fo] = F[c];
           if (want_flux && fout[0]) {
+            const int b = fo / (S.tx + 1), af = fo - b * (S.tx + 1);
             const int64_t nf = (int64_t)g.na + 1;
 #pragma unroll
             for (int c = 0; c < NV; ++c)
               if (c < nvo) fout[0][((int64_t)(c * g.np + it) * g.nb + (y0 + b)) * nf + x0 + af] = F[c];
           }
         } else {
-          const int a = i, bf = j;
 #pragma unroll
           for (int c = 0; c < NV; ++c)
-            if (TFV_IN(24, bf * S.tx + a, fb_plane)) fb[c * fb_plane + bf * S.tx + a] = F[c];
+            if (TFV_IN(24, fo, fb_plane)) fb[c * fb_plane + fo] = F[c];
           if (want_flux && fout[1]) {
+            const int bf = fo / S.tx, a = fo - bf * S.tx;
 #pragma unroll
             for (int c = 0; c < NV; ++c)
               if (c < nvo) fout[1][((int64_t)(c * g.np + it) * (g.nb + 1) + (y0 + bf)) * g.na + x0 + a] = F[c];
