@@ -5,7 +5,7 @@
 // pipe, so a packed instruction saves an issue slot; packing costs nothing
 // where the halves are results that the compiler can place side by side: the
 // two sides of a face, a cell's upper and lower predicted states.  3D step 256^3
-// 51.8 -> 49.0 warp instructions a cell, 986 -> 963 us a step; 32 2D grids of
+// 51.8 -> 49.0 warp instructions a cell, 986 -> 966 us a step; 32 2D grids of
 // 64^2 to 1024^2 499 -> 485 us.  Limited slopes of two components packed
 // (min / max have no packed form) were slower by 0.6%.
 #pragma once
