@@ -79,10 +79,14 @@ __device__ __forceinline__ void prim_from(const R* u, R g, R* p) {
 
 // Component v of a state array at cell offset `at`: the component's base is
 // uniform over the grid and the offset 32 bits (a component stays below 2^31
-// cells), which spares the 64-bit address arithmetic of every access.
+// cells), which spares the 64-bit address arithmetic of every access.  An
+// ordinary load: a launch of these kernels may begin before the kernel that
+// writes this state has ended, so the state is not read-only for the kernel's
+// lifetime as a non-coherent load (ro) asks, and pdl_wait orders ordinary loads
+// only.  ro is for the geometry factors, written once at bind.
 template <typename R>
 __device__ __forceinline__ R row(const R* base, int64_t nc, int v, uint32_t at) {
-  return ro(base + v * nc + at);
+  return base[v * nc + at];
 }
 
 // Half slopes of a cell from its neighbours' primitives (cell_slope, halved).
