@@ -435,10 +435,10 @@ struct HydroTile {
   static __device__ __forceinline__ void copy_plane(const Geo<DIM>& g, const R* U, const R* gam,
                                                     R* dst, const HydroSmem<R, DIM, VARG>& S,
                                                     int x0, int y0, int ax, int by, int p) {
-    const int la0 = x0 == 0 ? 2 : 0;  // staged columns and rows inside the domain
-    const int cols = min(ax + 4, g.na - x0 + 2) - la0;
-    const int lb0 = DIM == 3 && y0 == 0 ? 2 : 0;
-    const int rows = (DIM == 3 ? min(by + 4, g.nb - y0 + 2) : 1) - lb0;
+    const int la0 = halo_before(x0);  // staged columns and rows inside the domain
+    const int cols = ax + 4 - la0 - halo_after(x0, ax, g.na);
+    const int lb0 = DIM == 3 ? halo_before(y0) : 0;
+    const int rows = DIM == 3 ? by + 4 - lb0 - halo_after(y0, by, g.nb) : 1;
     const int64_t base = (int64_t)p * g.ps + (DIM == 3 ? (int64_t)(y0 - 2) * g.na : 0) + (x0 - 2);
     if constexpr (sizeof(R) == 4) {
       // pairs: every address even (8 bytes), rows of whole pairs
@@ -478,16 +478,16 @@ struct HydroTile {
   }
 
   // After the copy of an in-range plane: write the in-plane ghost cells
-  // (outside the domain; zero-filled by a tensor copy) by the boundary rules.  Only tiles touching an in-plane domain edge have any.
+  // (outside the domain; zero-filled by a tensor copy) by the boundary rules.
+  // Only tiles within two cells of an in-plane domain edge have any.
   static __device__ __forceinline__ void fix_ghosts(const InstDesc& d, const Geo<DIM>& g,
                                                     const R* U, const R* gam, R* dst,
                                                     const HydroSmem<R, DIM, VARG>& S, int x0,
                                                     int y0, int ax, int by, int p) {
     const int H = DIM == 3 ? by + 4 : 1;
-    const int aL = x0 == 0 ? 2 : 0;
-    const int aR = max(0, x0 + ax + 2 - g.na);
-    const int bL = (DIM == 3 && y0 == 0) ? 2 : 0;
-    const int bR = DIM == 3 ? max(0, y0 + by + 2 - g.nb) : 0;
+    const int aL = halo_before(x0), aR = halo_after(x0, ax, g.na);
+    const int bL = DIM == 3 ? halo_before(y0) : 0;
+    const int bR = DIM == 3 ? halo_after(y0, by, g.nb) : 0;
     const int wm = ax + 4 - aL - aR;
     const int n1 = (aL + aR) * H;  // ghost columns, every row
     const int n2 = (bL + bR) * wm; // ghost rows, the other columns
@@ -771,8 +771,9 @@ __device__ bool hydro_tile(const StepArgs& A, int t, unsigned char* smem,
   // one cp.async.bulk.tensor per plane (plus one for gamma), of another
   // instance by one cp.async per cell; ghost planes use plain loads.
   const bool use_tma = d.tma != 0;
-  const bool edge_tile = x0 == 0 || x0 + ax + 2 > g.na ||
-                         (DIM == 3 && (y0 == 0 || y0 + by + 2 > g.nb));
+  const bool edge_tile =
+      halo_before(x0) > 0 || halo_after(x0, ax, g.na) > 0 ||
+      (DIM == 3 && (halo_before(y0) > 0 || halo_after(y0, by, g.nb) > 0));
   const char* maps = reinterpret_cast<const char*>(A.tmaps) + (size_t)T.inst * 4 * 128;
   const void* map_u = maps + src * 128;
   const void* map_g = maps + 3 * 128;
