@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "tfv.h"
+#include "tfv_fork.h"
 #include "tfv_launch.h"
 #include "tfv_types.h"
 
@@ -537,20 +538,29 @@ cudaError_t launch_range_unchecked(tfv_batch* b, int op, int lim, int t0, int t1
 cudaError_t launch(tfv_batch* b, int op, int src_off, int dst_off) {
   if (op != kOpHydro)
     return launch_range(b, op, 0, 0, (int)b->tiles.size(), src_off, dst_off, b->stream);
-  const bool forked = !b->side.empty();
-  cudaError_t e = forked ? cudaEventRecord(b->fork, b->stream) : cudaSuccess;
-  for (size_t k = 0; k < b->groups.size() && e == cudaSuccess; ++k) {
+  auto group = [&](int k, cudaStream_t s) {
     const auto& g = b->groups[k];
-    const bool own = forked && k > 0;
-    cudaStream_t s = own ? b->side[k - 1] : b->stream;
-    if (own) e = cudaStreamWaitEvent(s, b->fork, 0);
-    if (e == cudaSuccess)
-      e = launch_range(b, op, g.limiter, g.t_begin, g.t_end, src_off, dst_off, s);
-    if (own && e == cudaSuccess) e = cudaEventRecord(b->join[k - 1], s);
+    return launch_range(b, op, g.limiter, g.t_begin, g.t_end, src_off, dst_off, s);
+  };
+  const int n = (int)b->groups.size();
+  if (b->side.empty()) {
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < n && e == cudaSuccess; ++k) e = group(k, b->stream);
+    return e;
   }
-  for (size_t k = 0; forked && k < b->side.size() && e == cudaSuccess; ++k)
-    e = cudaStreamWaitEvent(b->stream, b->join[k], 0);
-  return e;
+  struct Streams {
+    tfv_batch* b;
+    cudaError_t fork() { return cudaEventRecord(b->fork, b->stream); }
+    cudaError_t enter(int k) { return cudaStreamWaitEvent(b->side[k - 1], b->fork, 0); }
+    cudaError_t leave(int k) {
+      const cudaError_t e = cudaEventRecord(b->join[k - 1], b->side[k - 1]);
+      return e == cudaSuccess ? cudaStreamWaitEvent(b->stream, b->join[k - 1], 0) : e;
+    }
+    void drain(int k) { cudaStreamSynchronize(b->side[k - 1]); }
+  } streams{b};
+  return fork_join<cudaError_t>(streams, n, [&](int k) {
+    return group(k, k > 0 ? b->side[k - 1] : b->stream);
+  });
 }
 
 void drop_side_streams(tfv_batch* b) {
