@@ -152,7 +152,10 @@ MArgs<R> make_args(const tfv_metric* m) {
   A.err = reinterpret_cast<int32_t*>(m->ws + m->off_err);
   if (m->tiled) {
     A.cfl = m->cfg.cfl;
-    A.igm1 = (R)(1.0 / (m->cfg.gamma - 1.0));
+    // the inverse of what the kernels multiply by, gamma - 1 formed in R: from the
+    // unrounded gamma, energies of face states would not match the cells they come
+    // from (gamma 1.0001 in single precision: by 1.7e-4)
+    A.igm1 = R(1) / (A.gam - R(1));
     A.ntx = m->ntx;
     A.nty = m->nty;
   }
