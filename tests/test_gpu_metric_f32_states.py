@@ -48,3 +48,16 @@ def test_gamma_close_to_one(counts):
         s64.step()
         s32.step()
     assert max(errors(s64, s32)) <= 1e-5
+
+
+@pytest.mark.parametrize("limiter", ["VanLeer", "MINBEE", "Superbee", "Unos"])
+@pytest.mark.parametrize("counts", [(32, 24), (32, 24, 16)])
+def test_pressures_of_1e20(counts, limiter):
+    """Differences of neighbouring pressures around 1e19 to 1e20, whose product is
+    beyond single precision: slopes stay finite and the step second order."""
+    s64, s32 = sessions(stream(counts, 3e20, 1e9), limiter=limiter)
+    for _ in range(4):
+        s64.step()
+        s32.step()
+    assert s64.fallback_steps == 0 and s32.fallback_steps == 0
+    assert max(errors(s64, s32)) <= 1e-5

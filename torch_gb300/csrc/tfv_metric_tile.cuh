@@ -89,13 +89,28 @@ __device__ __forceinline__ R row(const R* base, int64_t nc, int v, uint32_t at) 
   return base[v * nc + at];
 }
 
+// Limited slope of one component (metric_limited).  Single-precision VanLeer,
+// 2 minus plus / (minus + plus), takes the quotient first: the Cartesian step's
+// product of the differences overflows where both exceed 1.8e19 (pressures in
+// small units), and the infinite slope would cost the step its second order.
+template <typename R, int LIM>
+__device__ __forceinline__ R tile_slope(R m, R c, R p) {
+  if constexpr (!Exact<R>::value && LIM == 0) {
+    const R minus = c - m, plus = p - c;
+    const R mp = minus * plus;  // its sign, and NaN for NaN
+    const R v = (minus + minus) * (plus * rcp(minus + plus));
+    return mp > R(0) ? v : (mp == mp ? R(0) : mp);
+  }
+  return limited_slope<R, 3, LIM>(m, c, p);
+}
+
 // Half slopes of a cell from its neighbours' primitives (cell_slope, halved).
 template <typename R, int NV, int LIM>
 __device__ __forceinline__ void half_slopes(const R* m, const R* c, const R* p, R* h) {
   R s0 = R(0), s1 = R(0);
 #pragma unroll
   for (int v = 0; v < NV; ++v) {
-    const R s = limited_slope<R, 3, LIM>(m[v], c[v], p[v]);
+    const R s = tile_slope<R, LIM>(m[v], c[v], p[v]);
     h[v] = hf(s);
     if (v == 0) s0 = h[v];
     if (v == NV - 1) s1 = h[v];
