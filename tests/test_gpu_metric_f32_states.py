@@ -50,7 +50,7 @@ def test_gamma_close_to_one(counts):
     assert max(errors(s64, s32)) <= 1e-5
 
 
-@pytest.mark.parametrize("limiter", ["VanLeer", "MINBEE", "Superbee", "Unos"])
+@pytest.mark.parametrize("limiter", ["VanLeer", "Albada", "MINBEE", "Superbee", "Unos"])
 @pytest.mark.parametrize("counts", [(32, 24), (32, 24, 16)])
 def test_pressures_of_1e20(counts, limiter):
     """Differences of neighbouring pressures around 1e19 to 1e20, whose product is

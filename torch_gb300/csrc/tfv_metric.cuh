@@ -268,7 +268,8 @@ __device__ __forceinline__ R metric_limited(R minus, R plus, int lim) {
   if (lim == 0) {
     phi = (R(2) * pos) / (R(1) + pos);
   } else if (lim == 1) {
-    phi = (pos * pos + pos) / (pos * pos + R(1));
+    const R q = np_min(pos, R(1e18));  // phi is 1 long before; its square is finite
+    phi = (q * q + q) / (q * q + R(1));
   } else if (lim == 2) {
     phi = np_max(R(0), np_min(r, R(1)));
   } else if (lim == 3) {

@@ -202,8 +202,8 @@ __device__ __forceinline__ R limited_slope(R um, R uc, R up) {
   R phi;
   if constexpr (Exact<R>::value) {
     phi = limiter_phi<DIM, LIM>(r);
-  } else if (LIM == 1) {  // Albada
-    const R pos = np_max(r, R(0));
+  } else if (LIM == 1) {  // Albada; phi is 1 long before the bound, r^2 finite up to it
+    const R pos = np_min(np_max(r, R(0)), R(1e18));
     phi = dv(pos * pos + pos, pos * pos + R(1));
     if (DIM == 2 && !(r > R(0))) phi = R(0);
   } else {  // Unos (MINBEE, Superbee and VanLeer returned above)
