@@ -132,41 +132,6 @@ __device__ __forceinline__ float desc_gamma(const D& d, float) { return d.gamma_
 // 2D: python/cfdSolver/torchSolver2D.py:124-168 (VanLeer/Albada zero for
 //     r <= 0, Unos without the (1+2r)/3 bound).
 // --------------------------------------------------------------------------
-// phi(r) in double precision, region by region: the numpy.maximum /
-// numpy.minimum nests of the reference reduce to comparisons of r with
-// constants whose low word is zero, decided by r's high word, and each region
-// returns the nest's value bit for bit (zeros with their sign, NaN for NaN).
-template <int DIM, int LIM>
-__device__ __forceinline__ double limiter_phi(double r) {
-  const uint32_t h = s64_hi(r), l = s64_lo(r);
-  const bool nan = soft_isnan(r);
-  const bool zero = ((h << 1) | l) == 0u;
-  const bool pos = (int32_t)h >= 0 && !zero;  // r > 0 (NaN apart)
-  double phi;
-  if (LIM == 0) {  // VanLeer: 2 pos / (1 + pos), pos = max(r, 0)
-    phi = soft_div(soft_twice(r), 1.0 + r);
-    if (!pos) phi = (DIM == 3 && zero) ? r : 0.0;  // max(-0, 0) is -0
-  } else if (LIM == 1) {  // Albada: (pos^2 + pos) / (pos^2 + 1)
-    const double q = r * r;
-    phi = soft_div(q + r, q + 1.0);
-    if (!pos) phi = 0.0;
-  } else if (LIM == 2) {  // MINBEE: max(0, min(r, 1))
-    phi = h < 0x3ff00000u ? r : 1.0;
-    if (!pos) phi = 0.0;
-  } else if (LIM == 3) {  // Superbee: max(0, max(min(2r, 1), min(r, 2)))
-    phi = h < 0x40000000u ? r : 2.0;
-    if (h < 0x3ff00000u) phi = h < 0x3fe00000u ? soft_twice(r) : 1.0;
-    if (!pos) phi = 0.0;
-  } else {  // Unos: max(0, min(min(2, 2r), (2 + r) / 3 [, (1 + 2r) / 3 in 3D]))
-    const double r2 = soft_twice(r);
-    const double m = h >= 0x3ff00000u ? 2.0 : r2;
-    const double a = soft_div(2.0 + r, 3.0);
-    phi = DIM == 3 ? soft_min(soft_min(m, a), soft_div(1.0 + r2, 3.0)) : soft_min(m, a);
-    if (!pos) phi = 0.0;
-  }
-  return nan ? r : phi;
-}
-
 template <typename R, int DIM, int LIM>
 __device__ __forceinline__ R limited_slope(R um, R uc, R up) {
   const R minus = uc - um;
