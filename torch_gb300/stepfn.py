@@ -29,8 +29,10 @@ def _device():
 
 def _as_device(x, dtype, device):
     # the transfer to the device copies a plain array; others (reversed, read-only,
-    # strided) become one first
-    if isinstance(x, np.ndarray) and not (x.flags.c_contiguous and x.flags.writeable):
+    # strided) become one first.  A reversed axis of one cell leaves an array
+    # contiguous with a negative stride, which torch refuses
+    if isinstance(x, np.ndarray) and not (x.flags.c_contiguous and x.flags.writeable
+                                          and min(x.strides, default=0) >= 0):
         x = np.array(x, copy=True)
     return torch.as_tensor(x, dtype=dtype, device=device).contiguous()
 
