@@ -140,6 +140,11 @@ int tfv_batch_create(int32_t dim, int32_t precision, int32_t n, const tfv_config
  * per-tile partials, scalars, 1D scratch). */
 int tfv_batch_workspace_size(const tfv_batch* b, size_t* bytes);
 
+/* Tile of the batch: the caller's, or the library's own choice where
+ * tfv_batch_create got none.  Creating a batch of the same instances with it
+ * gives the same tiling. */
+int tfv_batch_tile(const tfv_batch* b, tfv_tile* tile);
+
 /* Number of state buffers each instance needs in its ring (2, or 3 when
  * reactive). */
 int tfv_batch_ring_size(const tfv_batch* b, int32_t* nring);

@@ -107,6 +107,7 @@ _SIGS = {
     "tfv_batch_create": ([C.c_int32, C.c_int32, C.c_int32, C.POINTER(Config), C.POINTER(Tile),
                           C.POINTER(_VP)], C.c_int),
     "tfv_batch_workspace_size": ([_VP, C.POINTER(C.c_size_t)], C.c_int),
+    "tfv_batch_tile": ([_VP, C.POINTER(Tile)], C.c_int),
     "tfv_batch_ring_size": ([_VP, C.POINTER(C.c_int32)], C.c_int),
     "tfv_batch_bind": ([_VP, _VP, C.POINTER(_VP), C.POINTER(_VP), C.POINTER(_VP), _VP], C.c_int),
     "tfv_batch_advance": ([_VP, C.c_int32], C.c_int),

@@ -1,10 +1,11 @@
 """Tile-shape autotuner for the batched step.
 
 For a set of grids, time a few steps of every candidate tile configuration
-(in-plane tile shape, marching chunk, one CTA per tile or a persistent grid)
-on scratch copies of the grids, and return the fastest.  Results are cached
-per GPU, dimension, precision and grid-size signature in
-``$TORCH_GB300_CACHE`` (default ``~/.cache/torch_gb300/autotune.json``).
+(the library's own choice first, then in-plane tile shapes, marching chunks, one
+CTA per tile or a persistent grid) on scratch copies of the grids, and return
+the fastest.  Results are cached per GPU, library sources, dimension, precision
+and the grids' sizes, limiters and chemistry in ``$TORCH_GB300_CACHE`` (default
+``~/.cache/torch_gb300/autotune.json``).
 """
 
 import copy
@@ -15,7 +16,8 @@ from pathlib import Path
 
 import torch
 
-from .batch import Batch
+from . import build as _build
+from .batch import Batch, default_tile
 
 CACHE = Path(os.environ.get("TORCH_GB300_CACHE",
                             Path.home() / ".cache" / "torch_gb300" / "autotune.json"))
@@ -47,10 +49,21 @@ def candidates(dim, precision, sms):
 
 def signature(grids):
     g0 = grids[0]
-    sizes = sorted(tuple(g.counts) for g in grids)
-    key = json.dumps([torch.cuda.get_device_name(g0.device), g0.dim, g0.precision,
-                      sizes, [bool(g.reactive) for g in grids]])
+    # what a step's time depends on, and the sources whose kernels were timed
+    # beside which candidates
+    work = sorted([*g.counts, g.cfg.limiter, int(g.reactive), g.cfg.kinetic_model, g.cfg.closure]
+                  for g in grids)
+    key = json.dumps([torch.cuda.get_device_name(g0.device), _sources(), g0.dim, g0.precision,
+                      work])
     return hashlib.sha1(key.encode()).hexdigest()
+
+
+def _sources():
+    """Digest of the kernel sources and of this file."""
+    h = hashlib.sha1()
+    for p in sorted(_build.CSRC.glob("*")) + [Path(_build.__file__), Path(__file__)]:
+        h.update(p.read_bytes())
+    return h.hexdigest()
 
 
 def _load_cache():
@@ -101,7 +114,9 @@ def tune(grids, steps=4, warmup=2, use_cache=True, verbose=False):
         return tuple(cache[key]["tile"])
     sms = torch.cuda.get_device_properties(grids[0].device).multi_processor_count
     best, best_ms, results = None, float("inf"), []
-    for tile in candidates(grids[0].dim, grids[0].precision, sms):
+    own = default_tile(grids)
+    tried = candidates(grids[0].dim, grids[0].precision, sms)
+    for tile in [own] + [t for t in tried if t != own]:
         try:
             ms = time_config(grids, tile, steps, warmup)
         except (RuntimeError, ValueError):

@@ -119,6 +119,20 @@ class Grid:
         return self.current.detach().to("cpu", torch.float64).numpy()
 
 
+def default_tile(grids):
+    """Tile (tx, ty, chunk, persistent_ctas, tma) that a Batch of `grids` takes when
+    it is given none."""
+    lib = _lib.load()
+    cfgs = (_lib.Config * len(grids))(*[g.cfg for g in grids])
+    handle, tile = C.c_void_p(), _lib.Tile()
+    _lib.check(lib.tfv_batch_create(
+        grids[0].dim, _lib.TFV_FP64 if grids[0].precision == "fp64" else _lib.TFV_FP32,
+        len(grids), cfgs, None, C.byref(handle)))
+    _lib.check(lib.tfv_batch_tile(handle, C.byref(tile)))
+    _lib.check(lib.tfv_batch_destroy(handle))
+    return tile.tx, tile.ty, tile.chunk, tile.persistent_ctas, tile.tma
+
+
 class Batch:
     """Advance a list of grids of one dimension and precision together."""
 

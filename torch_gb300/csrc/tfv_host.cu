@@ -699,7 +699,27 @@ static int device_sms() {
   return sms;
 }
 
-// Tile of a double-precision 2D / 3D batch: the shape and chunk of the list
+// Tile shapes of the library's own choice whose cells leave lanes of the CTA to
+// the ring cells (double precision) or to the halo (1D).  A caller may name
+// them too (the autotuner returns them); any other shape that is not whole warps
+// keeps to step_threads.
+struct OwnShape {
+  int dim, tx, ty, threads;
+};
+static const OwnShape kOwnF64[] = {
+    {2, 30, 1, 32}, {2, 62, 1, 64}, {2, 126, 1, 128}, {3, 10, 8, 128}, {3, 14, 14, 256}};
+static const OwnShape kOwn1d = {1, 122, 1, 128};
+
+// Threads of a CTA for a tile: a shape of the library's own, else step_threads.
+static int tile_threads(int dim, int32_t precision, int tx, int ty) {
+  if (dim == 1 && tx == kOwn1d.tx) return kOwn1d.threads;
+  if (precision == TFV_FP64)
+    for (const OwnShape& S : kOwnF64)
+      if (S.dim == dim && S.tx == tx && S.ty == ty) return S.threads;
+  return step_threads(dim, precision == TFV_FP64, tx, ty);
+}
+
+// Tile of a double-precision 2D / 3D batch: the shape of kOwnF64 and the chunk
 // with the smallest modelled time.  Shapes leave lanes for the ring cells
 // (30 + 2, 62 + 2, 126 + 2 in 2D; 10 x 8 + 40 of 128 and 14 x 14 + 60 of 256
 // threads in 3D), so no warp does a second cell stage per plane; their widths
@@ -715,20 +735,13 @@ static int device_sms() {
 // whose 16 tiles leave most SMs idle), long ones on large grids (1024^2: 1.05
 // ms with 126 x 16, 1.26 with 30 x 4).
 static void fp64_tile(tfv_batch* b, const tfv_config* cfgs) {
-  struct Shape {
-    int tx, ty, threads;
-  };
-  static const Shape k2d[] = {{30, 1, 32}, {62, 1, 64}, {126, 1, 128}};
-  static const Shape k3d[] = {{10, 8, 128}, {14, 14, 256}};
   static const int kChunks[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
   const bool d3 = b->dim == 3;
-  const Shape* shapes = d3 ? k3d : k2d;
-  const int nshapes = d3 ? 2 : 3;
   const double sms = device_sms();
   const double stage = d3 ? 2.7 : 1.0, alpha = d3 ? 1.2 : 6.6, beta = d3 ? 1.18 : 0.95;
   double best = 0.0;
-  for (int k = 0; k < nshapes; ++k) {
-    const Shape& S = shapes[k];
+  for (const OwnShape& S : kOwnF64) {
+    if (S.dim != b->dim) continue;
     const double faces = double((S.tx + 1) * S.ty + (d3 ? S.tx * (S.ty + 1) : 0)) / S.threads;
     for (int c : kChunks) {
       double tiles = 0.0;
@@ -745,7 +758,6 @@ static void fp64_tile(tfv_batch* b, const tfv_config* cfgs) {
         b->tile.tx = S.tx;
         b->tile.ty = S.ty;
         b->tile.chunk = c;
-        b->block = S.threads;
       }
     }
   }
@@ -810,8 +822,7 @@ static void default_tile(tfv_batch* b, const tfv_config* cfgs) {
     // thread in every phase of the step (256 cells in 256 threads took two
     // rounds: 16 tubes of 194k cells, FP32 40.1 -> 34.4 us per step, FP64 204 ->
     // 156; one 1000-cell tube, FP64 59.6 -> 38.6)
-    b->tile.tx = 122;
-    b->block = 128;
+    b->tile.tx = kOwn1d.tx;
   } else if (b->precision == TFV_FP64) {
     fp64_tile(b, cfgs);
   } else if (b->dim == 3) {
@@ -878,16 +889,16 @@ static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_
     }
   }
   if (b->tile.tx < 4 || b->tile.ty < 1 || b->tile.chunk < 1 || b->tile.tx * b->tile.ty > 256 ||
-      (tile && step_threads(dim, precision == TFV_FP64, b->tile.tx, b->tile.ty) % 32 != 0)) {
+      tile_threads(dim, precision, b->tile.tx, b->tile.ty) % 32 != 0) {
     delete b;
     return fail(TFV_EINVAL,
                 "tile shape must have tx >= 4, ty >= 1, chunk >= 1, at most 256 cells, and "
                 "tx*ty a multiple of 32 (single precision: tx*ty plus its ring cells within "
-                "whole warps of at most 256 threads)");
+                "whole warps of at most 256 threads), or be a shape the library picks itself");
   }
   // every kernel of the batch runs whole warps (the block reductions shuffle
   // over full warps); lanes past a tile's cells own nothing
-  if (b->block == 0) b->block = step_threads(dim, precision == TFV_FP64, b->tile.tx, b->tile.ty);
+  b->block = tile_threads(dim, precision, b->tile.tx, b->tile.ty);
   b->reactive = cfgs[0].reactive != 0;
   // reactive SI closure: gamma(lambda) per cell, computed into the workspace
   b->own_gamma = b->reactive && cfgs[0].closure == TFV_CLOSURE_SI;
@@ -906,6 +917,12 @@ static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_
 int tfv_batch_workspace_size(const tfv_batch* b, size_t* bytes) {
   if (!b || !bytes) return fail(TFV_EINVAL, "invalid arguments");
   *bytes = b->total;
+  return TFV_OK;
+}
+
+int tfv_batch_tile(const tfv_batch* b, tfv_tile* tile) {
+  if (!b || !tile) return fail(TFV_EINVAL, "invalid arguments");
+  *tile = b->tile;
   return TFV_OK;
 }
 
