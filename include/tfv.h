@@ -216,7 +216,8 @@ int tfv_hllc_flux(int32_t precision, int32_t nv, int64_t n, const void* ul, cons
  * torchSolver3D.py:122-203): state_in -> state_out with the given dt and
  * per-cell gamma (NULL: cfg->gamma).  Writes face fluxes when fx/fy/fz are
  * non-NULL and *used_fallback.  Synchronous; needs a workspace of
- * tfv_step_workspace_size bytes. */
+ * tfv_step_workspace_size bytes (a bound over the plans that the step may make
+ * for the grid, with a per-cell gamma and without). */
 int tfv_step_workspace_size(const tfv_config* cfg, int32_t precision, size_t* bytes);
 int tfv_hydro_step(const tfv_config* cfg, int32_t precision, const void* state_in,
                    void* state_out, const void* gamma_cells, double dt, void* fx, void* fy,
@@ -231,8 +232,8 @@ int tfv_hydro_step(const tfv_config* cfg, int32_t precision, const void* state_i
  * The step's scratch (descriptors, tile table, per-tile partial sums, and
  * per-cell interface data of 1D tubes) lives in a 1 MiB array inside the
  * library's device image; every GPU that loads the library holds it until the
- * process exits.  A grid whose default tiles need more (tfv_step_workspace_size)
- * takes the largest tiles instead; grids whose scratch would not fit even so
+ * process exits.  A grid whose default tiles need more takes the largest tiles
+ * instead; grids whose scratch would not fit even so
  * are rejected with TFV_EINVAL (a 3D 256^3 grid needs about 376 KiB in fp32 and
  * 856 KiB in fp64 with the largest tiles, so
  * fp64 3D grids much larger than 256^3 are rejected; a 2D 4096^2 grid needs

@@ -151,9 +151,10 @@ void build_tiles(tfv_batch* b) {
   }
 }
 
-// Resident step-kernel CTAs on the current device (SMs x CTAs per SM), or 0
-// when no device is available or the launch is persistent.
-int resident_slots(const tfv_batch* b) {
+// Resident step-kernel CTAs on the current device (SMs x CTAs per SM) with or
+// without a per-cell gamma, or 0 when no device is available or the launch is
+// persistent.
+int resident_slots(const tfv_batch* b, bool varg) {
   if (b->dim == 1 || b->tile.persistent_ctas > 0) return 0;
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -164,11 +165,11 @@ int resident_slots(const tfv_batch* b) {
   const bool f64 = b->precision == TFV_FP64;
   int per_sm = 0;
   if (b->dim == 3)
-    per_sm = f64 ? occupancy3_f64(b->varg, b->tile.tx, b->tile.ty, b->block)
-                 : occupancy3_f32(b->varg, b->tile.tx, b->tile.ty, b->block);
+    per_sm = f64 ? occupancy3_f64(varg, b->tile.tx, b->tile.ty, b->block)
+                 : occupancy3_f32(varg, b->tile.tx, b->tile.ty, b->block);
   else
-    per_sm = f64 ? occupancy2_f64(b->varg, b->tile.tx, b->block)
-                 : occupancy2_f32(b->varg, b->tile.tx, b->block);
+    per_sm = f64 ? occupancy2_f64(varg, b->tile.tx, b->block)
+                 : occupancy2_f32(varg, b->tile.tx, b->block);
   cudaGetLastError();
   return per_sm > 0 ? per_sm * sms : 0;
 }
@@ -197,9 +198,17 @@ double dispatch_makespan(const std::vector<double>& dur, int slots) {
 // resident CTAs partly idle, split the final `slots` tiles along the
 // marching axis into halves, so that the tail is made of short tiles.  The
 // split is kept only where the dispatch model predicts a shorter launch.
-void split_tail(tfv_batch* b) {
-  const int slots = resident_slots(b);
-  if (slots <= 0 || b->dim == 1) return;
+// A workspace is sized without the model, which costs 0.1 ms per 2,000 tiles:
+// kTailAll splits wherever the step could, with a per-cell gamma or without
+// (their kernels' resident CTAs differ), and so bounds every plan from above;
+// kTailNone bounds them from below.
+enum class Tail { kPlan, kAll, kNone };
+void split_tail(tfv_batch* b, Tail tail) {
+  if (b->dim == 1 || tail == Tail::kNone) return;
+  const int slots = tail == Tail::kPlan
+                        ? resident_slots(b, b->varg)
+                        : std::max(resident_slots(b, false), resident_slots(b, true));
+  if (slots <= 0) return;
   const int tx = b->tile.tx, ty = b->dim == 3 ? b->tile.ty : 1;
   auto weight = [&](const Tile& t) {
     const InstDesc& d = b->desc[t.inst];
@@ -213,7 +222,7 @@ void split_tail(tfv_batch* b) {
   for (const auto& g : b->groups) {
     std::vector<double> plain, split;
     const int first_split = std::max(g.t_begin, g.t_end - slots);
-    for (int t = g.t_begin; t < g.t_end; ++t) {
+    for (int t = g.t_begin; t < g.t_end && tail == Tail::kPlan; ++t) {
       const Tile& T = b->tiles[t];
       plain.push_back(weight(T));
       if (t >= first_split && T.p1 - T.p0 >= 8) {
@@ -225,7 +234,8 @@ void split_tail(tfv_batch* b) {
         split.push_back(weight(T));
       }
     }
-    const bool use = dispatch_makespan(split, slots) < 0.99 * dispatch_makespan(plain, slots);
+    const bool use = tail == Tail::kAll || dispatch_makespan(split, slots) <
+                                               0.99 * dispatch_makespan(plain, slots);
     for (int t = g.t_begin; t < g.t_end; ++t) {
       const Tile& T = b->tiles[t];
       if (use && t >= first_split && T.p1 - T.p0 >= 8) {
@@ -680,7 +690,8 @@ const char* tfv_version(void) {
 const char* tfv_last_error(void) { return g_error.c_str(); }
 
 static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_config* cfgs,
-                           const tfv_tile* tile, bool varg, tfv_batch** out);
+                           const tfv_tile* tile, bool varg, tfv_batch** out,
+                           Tail tail = Tail::kPlan);
 
 int tfv_batch_create(int32_t dim, int32_t precision, int32_t n, const tfv_config* cfgs,
                      const tfv_tile* tile, tfv_batch** out) {
@@ -846,7 +857,7 @@ static tfv_tile compact_tile(int32_t dim, int32_t precision) {
 }
 
 static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_config* cfgs,
-                           const tfv_tile* tile, bool varg, tfv_batch** out) {
+                           const tfv_tile* tile, bool varg, tfv_batch** out, Tail tail) {
   if (!out || !cfgs || n < 1) return fail(TFV_EINVAL, "invalid arguments");
   if (dim < 1 || dim > 3) return fail(TFV_EINVAL, "dimension must be 1, 2 or 3");
   if (precision != TFV_FP64 && precision != TFV_FP32) return fail(TFV_EINVAL, "bad precision");
@@ -907,7 +918,7 @@ static int create_internal(int32_t dim, int32_t precision, int32_t n, const tfv_
   b->desc.resize(n);
   for (int i = 0; i < n; ++i) fill_desc(b, i);
   build_tiles(b);
-  split_tail(b);
+  split_tail(b, tail);
   layout(b);
   b->st.assign(n, InstState{});
   *out = b;
@@ -1273,25 +1284,41 @@ static tfv_config single_step_config(const tfv_config* cfg) {
   return c;
 }
 
-static int step_workspace(const tfv_config* cfg, int32_t precision, const tfv_tile* tile,
-                          size_t* bytes) {
-  // with and without a per-cell gamma: the tail split of the tiles follows the
-  // resident CTAs of the kernel, which differ between the two
-  tfv_config c = single_step_config(cfg);
-  *bytes = 0;
+static int plan_bytes(const tfv_config* c, int32_t precision, const tfv_tile* tile, bool varg,
+                      Tail tail, size_t* bytes) {
+  tfv_batch* b = nullptr;
+  const int r = create_internal(c->dim, precision, 1, c, tile, varg, &b, tail);
+  if (r) return r;
+  *bytes = b->total;
+  tfv_batch_destroy(b);
+  return TFV_OK;
+}
+
+// Whether a step's plan, with a per-cell gamma or without, fits `limit` bytes:
+// the bounds decide where they can, the plans themselves in between.
+static int step_fits(const tfv_config* cfg, int32_t precision, const tfv_tile* tile, size_t limit,
+                     bool* fits, size_t* need) {
+  const tfv_config c = single_step_config(cfg);
+  int r = plan_bytes(&c, precision, tile, false, Tail::kNone, need);
+  if (r) return r;
+  *fits = false;
+  if (*need > limit) return TFV_OK;
+  size_t bytes = 0;
+  if ((r = plan_bytes(&c, precision, tile, false, Tail::kAll, &bytes))) return r;
+  *fits = bytes <= limit;
+  if (*fits) return TFV_OK;
   for (const bool varg : {false, true}) {
-    tfv_batch* b = nullptr;
-    const int r = create_internal(cfg->dim, precision, 1, &c, tile, varg, &b);
-    if (r) return r;
-    *bytes = std::max(*bytes, b->total);
-    tfv_batch_destroy(b);
+    if ((r = plan_bytes(&c, precision, tile, varg, Tail::kPlan, &bytes))) return r;
+    *need = std::max(*need, bytes);
   }
+  *fits = *need <= limit;
   return TFV_OK;
 }
 
 int tfv_step_workspace_size(const tfv_config* cfg, int32_t precision, size_t* bytes) {
   if (!cfg || !bytes) return fail(TFV_EINVAL, "invalid arguments");
-  return step_workspace(cfg, precision, nullptr, bytes);
+  const tfv_config c = single_step_config(cfg);
+  return plan_bytes(&c, precision, nullptr, false, Tail::kAll, bytes);
 }
 
 static int hydro_step(const tfv_config* cfg, int32_t precision, const tfv_tile* tile,
@@ -1374,18 +1401,19 @@ extern "C" int tfv_hydro_step_static(const tfv_config* cfg, int32_t precision,
                                      void* fz, int32_t* used_fallback, void* stream) {
   if (!cfg) return fail(TFV_EINVAL, "invalid arguments");
   size_t need = 0;
-  int r = step_workspace(cfg, precision, nullptr, &need);
+  bool fits = false;
+  int r = step_fits(cfg, precision, nullptr, kStaticScratchBytes, &fits, &need);
   if (r) return r;
   // a grid whose default tiling asks for more scratch takes the largest tiles
   // (fewer of them; values do not depend on the tile shape)
   tfv_tile compact;
   const tfv_tile* tile = nullptr;
-  if (need > kStaticScratchBytes) {
+  if (!fits) {
     compact = compact_tile(cfg->dim, precision);
     tile = &compact;
-    if ((r = step_workspace(cfg, precision, tile, &need))) return r;
+    if ((r = step_fits(cfg, precision, tile, kStaticScratchBytes, &fits, &need))) return r;
   }
-  if (need > kStaticScratchBytes)
+  if (!fits)
     return fail(TFV_EINVAL, "this grid needs " + std::to_string(need) +
                                 " bytes of step scratch but tfv_hydro_step_static holds " +
                                 std::to_string(kStaticScratchBytes) +
