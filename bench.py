@@ -582,6 +582,16 @@ def error_summary(rows):
     return out
 
 
+def compared(what, rows):
+    """What the result line says of a list of comparisons: the summary, how many
+    there were and the one with the largest density error.  The rows themselves go to
+    standard error: with one row per request the line grew with every request that
+    fitted the time budget, past what its readers take."""
+    print(json.dumps({what: rows}), file=sys.stderr, flush=True)
+    return dict(error_summary(rows), compared=len(rows),
+                worst=max(rows, key=lambda r: r["l1_rho"]))
+
+
 def solve_alone(grid, chunk=64, graph_steps=16):
     """Advance one grid alone until it is done or has made its maximum steps:
     device milliseconds of the launches (CUDA events on its stream).  Steps
@@ -643,7 +653,7 @@ def batched_leg(steps=500, count=64, seed=4):
         s = Batch([g], graph_steps=10)
         seq64 += _timed(s.stream, lambda: s.advance(steps))
         s.refresh()
-        errors.append(state_errors(u32, g.current))
+        errors.append(dict(state_errors(u32, g.current), n=p.shape[-1]))
         s.close()
     del finals
     torch.cuda.empty_cache()
@@ -662,11 +672,7 @@ def batched_leg(steps=500, count=64, seed=4):
                                   "how": "each grid alone, all its steps timed"},
         "speedup_vs_sequential_fp32": seq32 / ms,
         "speedup_vs_sequential_fp64": seq64 / ms,
-        "fp32_vs_fp64": dict(error_summary(errors),
-                             per_grid_l1_rho=[e["l1_rho"] for e in errors],
-                             per_grid_l1_p=[e["l1_p"] for e in errors],
-                             per_grid_linf_rho=[e["linf_rho"] for e in errors],
-                             per_grid_linf_p=[e["linf_p"] for e in errors]),
+        "fp32_vs_fp64": compared("batched fp32_vs_fp64 per grid", errors),
         "latency": "every grid finishes with the batch: p50 = p99 = batch_ms",
     }
 
@@ -742,7 +748,7 @@ def served_leg(rates=(10.0, 30.0, 100.0, 300.0, 1000.0), count=128, budget_gib=3
                        "each alone, all their steps timed"}
             entry["speedup_vs_sequential_fp64"] = (upd / st["wall_s"]) / (
                 sub_upd / (seq64_ms * 1e-3))
-            entry["fp32_vs_fp64"] = dict(error_summary(errors), requests=errors,
+            entry["fp32_vs_fp64"] = dict(compared("served fp32_vs_fp64 per request", errors),
                                          served_equals_alone_fp32=f"{same}/{len(keep)}")
         out.append(entry)
     return {"workload": "served mix: 40% 1D tubes N~logU[1e3,1e5], 40% 2D N^2 N~U[128,1024], "
