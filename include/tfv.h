@@ -314,6 +314,10 @@ int tfv_metric_create(int32_t precision, const tfv_metric_config* cfg, const dou
                       tfv_metric** out);
 int tfv_metric_workspace_size(tfv_metric* m, size_t* bytes);
 
+/* How the session's step is tiled: tile[4] = threads along x and y of a block,
+ * planes it marches through, blocks; zeros where the separate kernels run. */
+int tfv_metric_tile(const tfv_metric* m, int32_t* tile);
+
 /* Attach the workspace (256-byte aligned) and the two state slots (and
  * lambda / beta slots of reactive sessions); slot 0 holds the initial state.
  * Computes the initial integral. */

@@ -97,6 +97,7 @@ _SIGS = {
     "tfv_metric_advance": ([_VP, C.c_int32], C.c_int),
     "tfv_metric_report": ([_VP, C.POINTER(Report)], C.c_int),
     "tfv_metric_integrals": ([_VP, C.POINTER(C.c_double)], C.c_int),
+    "tfv_metric_tile": ([_VP, C.POINTER(C.c_int32)], C.c_int),
     "tfv_metric_restore": ([_VP, C.POINTER(Report)], C.c_int),
     "tfv_metric_set_current": ([_VP, C.c_int32], C.c_int),
     "tfv_metric_destroy": ([_VP], C.c_int),

@@ -744,6 +744,13 @@ int tfv_metric_workspace_size(tfv_metric* m, size_t* bytes) {
   return TFV_OK;
 }
 
+int tfv_metric_tile(const tfv_metric* m, int32_t* tile) {
+  if (!m || !tile) return host_fail(TFV_EINVAL, "invalid arguments");
+  const int32_t t[4] = {m->bx, m->by, m->chunk, m->ntiles};
+  for (int k = 0; k < 4; ++k) tile[k] = m->tiled ? t[k] : 0;
+  return TFV_OK;
+}
+
 int tfv_metric_bind(tfv_metric* m, void* workspace, void* const* states, void* const* lams,
                     void* const* betas, void* stream) {
   if (!m || !workspace || !states || !states[0] || !states[1])
