@@ -123,9 +123,13 @@ inline TFV_HOST_DEVICE int step_threads(int dim, bool exact, int tx, int ty) {
 // A tile of `len` cells from cell `at` of an axis of `n` stages a two-cell halo
 // on either side: how many of the staged cells lie before the axis's first
 // cell (one, not none, for the second of two one-cell tiles) and after its last.
-inline TFV_HOST_DEVICE int halo_before(int at) { return at < 2 ? 2 - at : 0; }
+inline TFV_HOST_DEVICE int halo_before(int at) {
+  const int k = 2 - at;
+  return k > 0 ? k : 0;
+}
 inline TFV_HOST_DEVICE int halo_after(int at, int len, int n) {
-  return at + len + 2 > n ? at + len + 2 - n : 0;
+  const int k = at + len + 2 - n;
+  return k > 0 ? k : 0;
 }
 
 }  // namespace tfv
