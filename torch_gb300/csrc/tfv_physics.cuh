@@ -163,12 +163,15 @@ __device__ __forceinline__ R limited_slope(R um, R uc, R up) {
     const R v = (mp + mp) * rcp(minus + plus);
     return mp > R(0) ? v : (mp == mp ? R(0) : mp);
   }
-  const R r = dv(minus, guarded(plus, R(kGuard)));
+  // a divisor within the guard leaves |phi plus| below 1.2e-14 whatever stands in for
+  // it; in single precision a large one, so that Albada's r^2 stays finite (a
+  // pressure step of 5e5 Pa over 1e-14 does not)
+  const R r = dv(minus, abs_lt(plus, R(kGuard)) ? R(Exact<R>::value ? kGuard : 1e18) : plus);
   R phi;
   if constexpr (Exact<R>::value) {
     phi = limiter_phi<DIM, LIM>(r);
-  } else if (LIM == 1) {  // Albada; phi is 1 long before the bound, r^2 finite up to it
-    const R pos = np_min(np_max(r, R(0)), R(1e18));
+  } else if (LIM == 1) {  // Albada
+    const R pos = np_max(r, R(0));
     phi = dv(pos * pos + pos, pos * pos + R(1));
     if (DIM == 2 && !(r > R(0))) phi = R(0);
   } else {  // Unos (MINBEE, Superbee and VanLeer returned above)
