@@ -1617,7 +1617,7 @@ __device__ __forceinline__ bool react_cell(const Chem<R>& d, R* u, R& lam, R& be
 // (cur+1) and gamma(lambda) for the hydro step; wave maxima for the reactive
 // dt check (python/cfdSolver/torchSession.py:401-411).  Bound by HBM: the state
 // and the fractions read and written once, 48 B per cell in single precision.
-// A thread walks a column of its tile; the loads of kHeatPlanes planes are
+// A thread walks a column of its tile; the loads of HeatPlanes planes are
 // issued before the first is used (one plane at a time left the loop waiting
 // for memory: 192^3, 162 us a launch against 50 us of traffic; now 62).
 template <typename R>

@@ -2,13 +2,14 @@
 // and 3D in single precision: the CFL rate, and one SSPRK2 stage in a single
 // pass over the state.
 //
-// The separate kernels (tfv_metric.cuh; the other sessions keep them) write the primitives, the geometric source and every face flux of a
-// stage to HBM and read them back, about 150 B per cell and stage in single
-// precision.  Here a CTA owns a block of cells of the plane normal to the last
-// axis and marches along that axis through a chunk of planes: the primitives of
-// the current plane (with a two-cell halo) live in shared memory, the face
-// fluxes of the plane too, the marching-axis neighbours and the marching faces
-// in registers, and a stage reads the state once and writes it once.
+// The separate kernels (tfv_metric.cuh; the other sessions keep them) write the
+// primitives, the geometric source and every face flux of a stage to HBM and
+// read them back, about 150 B per cell and stage in single precision.  Here a
+// CTA owns a block of cells of the plane normal to the last axis and marches
+// along that axis through a chunk of planes: the primitives of the current
+// plane (with a two-cell halo) live in shared memory, the face fluxes of the
+// plane too, the marching-axis neighbours and the marching faces in registers,
+// and a stage reads the state once and writes it once.
 //
 // Work split.  Thread (a, b) of a BX x BY block forms its cell's limited slopes
 // once, leaves the cell's upper x and y face states in shared memory and then
@@ -24,14 +25,16 @@
 // Measured, 256 x 192 x 192 single precision: the two stages 571 and 611 us, the
 // rate 130 us, a step 1330; the separate kernels took 837 us a stage (march and
 // update 385, x faces 179, y faces 163, primitives 110) and 174 for the rate, a
-// step 2020 with its reductions and host looks.  Bound by instruction issue and latency: 1256 instructions a cell,
-// issue slots 52% busy from 16 warps per SM.  Variants: three CTAs per SM (84
-// registers) spill, a step 1650 us; high-edge faces by the column of threads
-// itself (no redundant slopes, one more barrier) 621 and 698 us.
+// step 2020 with its reductions and host looks.  Bound by instruction issue and
+// latency: 1256 instructions a cell, issue slots 52% busy from 16 warps per SM.
+// Variants: three CTAs per SM (84 registers) spill, a step 1650 us; high-edge
+// faces by the column of threads itself (no redundant slopes, one more barrier)
+// 621 and 698 us.
 //
 // Values are those of the separate kernels: in double precision bit for bit
 // (the same expressions in the same order), in single precision with
-// reciprocals shared and the division-free limiters of the Cartesian step.
+// reciprocals shared and the limiters of the Cartesian step but VanLeer
+// (tile_slope).
 //
 // Reference: python/cfdSolver/torchFiniteVolume.py:16-276.
 #pragma once

@@ -281,7 +281,6 @@ TFV_SOFT bool soft_ge0(double x) {
 TFV_SOFT bool soft_abs_lt(double x, double c) {
   return s64_join(s64_hi(x) & 0x7fffffffu, s64_lo(x)) < s64_join(s64_hi(c), s64_lo(c));
 }
-TFV_SOFT double soft_abs(double x) { return s64_make(s64_hi(x) & 0x7fffffffu, s64_lo(x)); }
 
 // numpy.maximum / numpy.minimum: NaN propagates, the first operand wins ties
 TFV_SOFT double soft_max(double a, double b) {
