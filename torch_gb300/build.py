@@ -6,8 +6,8 @@ Each translation unit is compiled by nvcc in parallel; the double-precision
 kernels are built with -fmad=false so that they keep NumPy's rounding, the
 single-precision kernels with FMA contraction, flush-to-zero and fast
 division/square root.  Output: torch_gb300/_build/libtfv.so; with --checked,
-the checked build torch_gb300/_build/checked/libtfv.so (kernel indexes
-tested against their buffers, for debugging).
+the checked build torch_gb300/_build/checked/libtfv.so (indexes of the
+hydrodynamic step tested against their buffers, for debugging).
 """
 
 import os
@@ -61,8 +61,9 @@ def _sources_newer(target):
 
 
 def library(checked=False):
-    """Path of the library: the release build, or the checked build (every
-    kernel index tested against its buffer, each launch waited for)."""
+    """Path of the library: the release build, or the checked build (the
+    hydrodynamic step's indexes tested against their buffers, each launch waited
+    for)."""
     return CHECKED_LIB if checked else LIB
 
 

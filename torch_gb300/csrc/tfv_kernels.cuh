@@ -71,10 +71,11 @@ __device__ __forceinline__ int map_axis(int i, int n, int bc, bool& ghost) {
 }
 
 // --------------------------------------------------------------------------
-// Checked build (TFV_CHECKED=1): every global and shared index of the step
-// kernels is tested against the extent of its buffer; the first violation is
-// recorded (site, block, index, extent) and the access is skipped.  The
-// record is per translation unit; the host reads it after each launch.
+// Checked build (TFV_CHECKED=1): the global and shared indexes of the
+// hydrodynamic step (not of the reaction and transport kernels) are tested
+// against the extents of their buffers; the first violation is recorded (site,
+// block, index, extent) and the access is skipped.  The record is per
+// translation unit; the host reads it after each launch.
 // --------------------------------------------------------------------------
 #if TFV_CHECKED
 static __device__ unsigned long long g_check[4];

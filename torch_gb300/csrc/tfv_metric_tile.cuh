@@ -26,7 +26,8 @@
 // rate 130 us, a step 1330; the separate kernels took 837 us a stage (march and
 // update 385, x faces 179, y faces 163, primitives 110) and 174 for the rate, a
 // step 2020 with its reductions and host looks.  Bound by instruction issue and
-// latency: 1256 instructions a cell, issue slots 52% busy from 16 warps per SM.
+// latency: 1261 instructions a cell, issue slots 51 to 56% busy from 16 warps per
+// SM.
 // Variants: three CTAs per SM (84 registers) spill, a step 1650 us; high-edge
 // faces by the column of threads itself (no redundant slopes, one more barrier)
 // 621 and 698 us.
